@@ -63,19 +63,110 @@ __global__ __launch_bounds__(kHistThreads) void hist_bytes_kernel(const uint8_t*
 // claimed one at a time (a claim held while another block is encoded would
 // stall every later block's look-back).
 // ------------------------------------------------------------------------
-// Four CTAs of eight warps per SM (32 warps, 64 registers a thread): with
-// five the register cap spills the pending block's state, which costs more
-// than the extra warps gain (0.695 vs 0.720 ms on 1 GiB of detector frames).
-constexpr int kEncMinCtas = 4;
+// One CTA of up to 32 warps per SM shares the 32 KiB table; small inputs take
+// smaller CTAs, so that their blocks spread over the SMs.
+constexpr int kEncMaxWarps = 32, kEncMaxThreads = kEncMaxWarps * 32;
 
-template <bool kSlots, bool kWide>
-__global__ __launch_bounds__(kEncThreads, kEncMinCtas) void ans_encode_kernel(
+// Empty input: header and a zero pdf only (GpuANSEncode.h:201-237).
+__device__ __forceinline__ void encode_empty(uint8_t* __restrict__ out, uint64_t out_cap, int p,
+                                             const uint32_t* __restrict__ pdf,
+                                             unsigned long long* out_size64, uint32_t* out_size32,
+                                             const Sink& sink, int lane) {
+  const uint64_t over = ans_overhead(0);
+  if (over > out_cap) {
+    if (lane == 0) report(sink, MANS_ERR_OUTPUT_OVERFLOW, over);
+    return;
+  }
+  if (lane < 8) {
+    const uint32_t hv = lane == 0 ? kAnsMagicVersion : (lane == 4 ? (uint32_t)p : 0u);
+    reinterpret_cast<uint32_t*>(out)[lane] = hv;
+  }
+  for (int i = lane; i < kAnsSyms; i += 32)
+    reinterpret_cast<uint16_t*>(out + kAnsHeaderBytes)[i] = (uint16_t)pdf[i];
+  if (lane == 0) {
+    if (out_size64) *out_size64 = over;
+    if (out_size32) *out_size32 = (uint32_t)over;
+  }
+}
+
+// The last CTA resets the work counters and advances the epoch: the call's
+// flags are then stale.
+__device__ __forceinline__ void encode_done(Ctrl* ctrl, uint32_t epoch) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&ctrl->done_counter[1], 1u) == gridDim.x - 1) {
+      ctrl->tile_counter[1] = 0;
+      ctrl->done_counter[1] = 0;
+      ctrl->epoch = (epoch + 1) & 0x3fffffffu;
+    }
+  }
+}
+
+template <int kP>
+__global__ __launch_bounds__(kEncMaxThreads, 1) void ans_encode_slots_kernel(
+    const uint8_t* __restrict__ in, uint8_t* __restrict__ out, uint64_t out_cap,
+    unsigned long long* out_size64, uint32_t* out_size32, Ctrl* ctrl, unsigned long long* flags,
+    uint8_t* __restrict__ slots) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  EncWarp& sw = reinterpret_cast<EncWarp*>(smem_raw + kEncTableBytes)[warp];
+  if (lane == 0) mbar_init(&sw.bar);
+  uint32_t parity = 0;
+  const Sink sink = sink_of(ctrl);
+  const bool failed = sink_failed(sink);
+  const uint32_t epoch = *((volatile uint32_t*)&ctrl->epoch);
+  const uint64_t n = __ldcg(&ctrl->merged_size);
+  const uint64_t nb = div_up_u64(n, kAnsBlock);
+  enc_fill_table(smem_raw, ctrl->enc_table, kP);
+  __syncthreads();
+  if (!failed && nb == 0 && blockIdx.x == 0 && warp == 0)
+    encode_empty(out, out_cap, kP, ctrl->pdf, out_size64, out_size32, sink, lane);
+
+  const uint32_t warps = blockDim.x >> 5, ahead = gridDim.x * warps;
+  // Two word slots per warp. A block's words wait in one slot for its
+  // stream offset while the warp encodes its next block into the other;
+  // the look-back of the waiting block then runs after that next block's
+  // aggregate is published, when its predecessors have usually finished,
+  // instead of stalling the warp. Every claimed block publishes its
+  // aggregate as soon as it is encoded, before any wait, so the deferred
+  // look-backs always complete.
+  uint16_t* const slot0 = reinterpret_cast<uint16_t*>(
+      slots + ((uint64_t)blockIdx.x * warps + warp) * 2 * kEncSlotBytes);
+  EncPending pend{0xffffffffu, 0, 0, nullptr};
+  uint32_t cur = 0;
+  while (!failed) {
+    const uint32_t b = warp_claim(&ctrl->tile_counter[1], lane);
+    if (b >= nb) break;
+    if (lane == 0 && (uint64_t)b + ahead < nb) {
+      const uint64_t s1 = ((uint64_t)b + ahead) * kAnsBlock;
+      prefetch_l2(in + s1, (uint32_t)min_u64(kAnsBlock, n - s1));
+    }
+    uint16_t* const sout = slot0 + cur * (kEncSlotBytes / 2);
+    uint32_t x;
+    const uint32_t nw = encode_words_rep<kP>(in, n, b, smem_raw, sw, parity, sout, sink, lane, x);
+    if (lane == 0)
+      st_flag(&flags[b], make_flag(b == 0 ? kFlagIncl : kFlagAgg, epoch, (nw + 7) & ~7u));
+    if (pend.b != 0xffffffffu)
+      encode_finish<true>(out, out_cap, n, out_size64, out_size32, ctrl->pdf, flags, epoch, kP,
+                          sink, pend, lane);
+    pend = EncPending{b, nw, x, sout};
+    cur ^= 1u;
+  }
+  if (pend.b != 0xffffffffu)
+    encode_finish<true>(out, out_cap, n, out_size64, out_size32, ctrl->pdf, flags, epoch, kP, sink,
+                        pend, lane);
+  encode_done(ctrl, epoch);
+}
+
+// The same with each block's words compacted in shared memory (no scratch in
+// global memory, no deferral), for the allocation-free call.
+__global__ __launch_bounds__(kEncThreads) void ans_encode_shared_kernel(
     const uint8_t* __restrict__ in, uint8_t* __restrict__ out, uint64_t out_cap,
     unsigned long long* out_size64, uint32_t* out_size32, Ctrl* ctrl,
-    unsigned long long* flags, int p, uint8_t* __restrict__ slots) {
+    unsigned long long* flags, int p) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
-  EncSmemSlots& ss = *reinterpret_cast<EncSmemSlots*>(smem_raw);  // common prefix of both layouts
-  __shared__ int s_last;
+  EncSmem& ss = *reinterpret_cast<EncSmem*>(smem_raw);
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   uint64_t* bar = &ss.bar[warp];
   if (lane == 0) mbar_init(bar);
@@ -85,118 +176,22 @@ __global__ __launch_bounds__(kEncThreads, kEncMinCtas) void ans_encode_kernel(
   const uint32_t epoch = *((volatile uint32_t*)&ctrl->epoch);
   const uint64_t n = __ldcg(&ctrl->merged_size);
   const uint64_t nb = div_up_u64(n, kAnsBlock);
-  const uint64_t over = ans_overhead(nb);
-  // Table layout: with a concentrated symbol distribution most lanes of a
-  // step look up the same few entries, and the expanded 16-byte entries save
-  // integer work; with a flat one the lanes spread over many entries, and
-  // the packed 8-byte entries cost fewer shared-memory wavefronts. The
-  // effective number of symbols 2^(2p) / sum(pdf^2) decides (<= 16:
-  // expanded). Both variants are launched; the one that does not match the
-  // table returns at once, before touching any counter. Either layout
-  // yields the same bytes.
-  __shared__ uint32_t s_sq[kEncWarps];
-  {
-    const uint32_t q = ctrl->pdf[t];
-    const uint32_t sq = __reduce_add_sync(0xffffffffu, q * q);
-    if (lane == 0) s_sq[warp] = sq;
-  }
+  if (!failed) ss.table[t] = ctrl->enc_table[t];
   __syncthreads();
-  uint64_t tot = 0;
-  for (int w = 0; w < kEncWarps; ++w) tot += s_sq[w];
-  if ((tot * 16ull >= (1ull << (2 * p))) != kWide) return;
-  if (!failed) {
-    if constexpr (kWide) ss.table4[t] = expand_enc_entry(ctrl->enc_table[t], p);
-    else ss.table2[t] = ctrl->enc_table[t];
-  }
-  __syncthreads();
-
-  if (!failed && nb == 0 && blockIdx.x == 0 && warp == 0) {
-    // Empty input: header and a zero pdf only (GpuANSEncode.h:201-237).
-    if (over > out_cap) {
-      if (lane == 0) report(sink, MANS_ERR_OUTPUT_OVERFLOW, over);
-    } else {
-      if (lane < 8) {
-        const uint32_t hv = lane == 0 ? kAnsMagicVersion : (lane == 4 ? (uint32_t)p : 0u);
-        reinterpret_cast<uint32_t*>(out)[lane] = hv;
-      }
-      for (int i = lane; i < kAnsSyms; i += 32)
-        reinterpret_cast<uint16_t*>(out + kAnsHeaderBytes)[i] = (uint16_t)ctrl->pdf[i];
-      if (lane == 0) {
-        if (out_size64) *out_size64 = over;
-        if (out_size32) *out_size32 = (uint32_t)over;
-      }
-    }
-  }
-
+  if (!failed && nb == 0 && blockIdx.x == 0 && warp == 0)
+    encode_empty(out, out_cap, p, ctrl->pdf, out_size64, out_size32, sink, lane);
   const uint32_t ahead = gridDim.x * kEncWarps;
-  if constexpr (kSlots) {
-    // Two word slots per warp. A block's words wait in one slot for its
-    // stream offset while the warp encodes its next block into the other;
-    // the look-back of the waiting block then runs after that next block's
-    // aggregate is published, when its predecessors have usually finished,
-    // instead of stalling the warp. Every claimed block publishes its
-    // aggregate as soon as it is encoded, before any wait, so the deferred
-    // look-backs always complete.
-    uint16_t* const slot0 = reinterpret_cast<uint16_t*>(
-        slots + ((uint64_t)blockIdx.x * kEncWarps + warp) * 2 * kEncSlotBytes);
-    EncPending pend{0xffffffffu, 0, 0, nullptr};
-    uint32_t cur = 0;
-    while (!failed) {
-      const uint32_t b = warp_claim(&ctrl->tile_counter[1], lane);
-      if (b >= nb) break;
-      if (lane == 0 && (uint64_t)b + ahead < nb) {
-        const uint64_t s1 = ((uint64_t)b + ahead) * kAnsBlock;
-        prefetch_l2(in + s1, (uint32_t)min_u64(kAnsBlock, n - s1));
-      }
-      uint16_t* const sout = slot0 + cur * (kEncSlotBytes / 2);
-      uint32_t x;
-      uint32_t nw;
-      if constexpr (kWide)
-        nw = encode_words<false>(in, n, b, ss.table4, ss.in[warp], bar, parity, sout, p, sink,
-                                 lane, x);
-      else
-        nw = encode_words<false>(in, n, b, ss.table2, ss.in[warp], bar, parity, sout, p, sink,
-                                 lane, x);
-      if (lane == 0)
-        st_flag(&flags[b], make_flag(b == 0 ? kFlagIncl : kFlagAgg, epoch, (nw + 7) & ~7u));
-      if (pend.b != 0xffffffffu)
-        encode_finish<true>(out, out_cap, n, out_size64, out_size32, ctrl->pdf, flags, epoch, p,
-                            sink, pend, lane);
-      pend = EncPending{b, nw, x, sout};
-      cur ^= 1u;
+  while (!failed) {
+    const uint32_t b = warp_claim(&ctrl->tile_counter[1], lane);
+    if (b >= nb) break;
+    if (lane == 0 && (uint64_t)b + ahead < nb) {
+      const uint64_t s1 = ((uint64_t)b + ahead) * kAnsBlock;
+      prefetch_l2(in + s1, (uint32_t)min_u64(kAnsBlock, n - s1));
     }
-    if (pend.b != 0xffffffffu)
-      encode_finish<true>(out, out_cap, n, out_size64, out_size32, ctrl->pdf, flags, epoch, p,
-                          sink, pend, lane);
-  } else {
-    uint16_t* sout = reinterpret_cast<EncSmem*>(smem_raw)->out[warp];
-    while (!failed) {
-      const uint32_t b = warp_claim(&ctrl->tile_counter[1], lane);
-      if (b >= nb) break;
-      if (lane == 0 && (uint64_t)b + ahead < nb) {
-        const uint64_t s1 = ((uint64_t)b + ahead) * kAnsBlock;
-        prefetch_l2(in + s1, (uint32_t)min_u64(kAnsBlock, n - s1));
-      }
-      if constexpr (kWide)
-        encode_block<false>(in, n, out, out_cap, out_size64, out_size32, ctrl->pdf, flags, epoch,
-                            p, sink, ss.table4, ss.in[warp], bar, parity, sout, b, lane);
-      else
-        encode_block<false>(in, n, out, out_cap, out_size64, out_size32, ctrl->pdf, flags, epoch,
-                            p, sink, ss.table2, ss.in[warp], bar, parity, sout, b, lane);
-    }
+    encode_block<false>(in, n, out, out_cap, out_size64, out_size32, ctrl->pdf, flags, epoch, p,
+                        sink, ss.table, ss.in[warp], bar, parity, ss.out[warp], b, lane);
   }
-
-  __syncthreads();
-  if (t == 0) {
-    __threadfence();
-    s_last = atomicAdd(&ctrl->done_counter[1], 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (s_last && t == 0) {
-    ctrl->tile_counter[1] = 0;
-    ctrl->done_counter[1] = 0;
-    ctrl->epoch = (epoch + 1) & 0x3fffffffu;  // the call's flags are now stale
-  }
+  encode_done(ctrl, epoch);
 }
 
 // ------------------------------------------------------------------------
@@ -296,22 +291,14 @@ static int occupancy(const void* fn, int threads, size_t smem) {
 }
 
 void init_ans_launch_cfg(LaunchCfg& cfg) {
-  cudaFuncSetAttribute(ans_encode_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  for (auto* k : {ans_encode_slots_kernel<9>, ans_encode_slots_kernel<10>, ans_encode_slots_kernel<11>})
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)enc_smem_bytes(kEncMaxWarps));
+  cudaFuncSetAttribute(ans_encode_shared_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(EncSmem));
-  cudaFuncSetAttribute(ans_encode_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(EncSmem));
+  cfg.enc_ctas = occupancy((const void*)ans_encode_shared_kernel, kEncThreads, sizeof(EncSmem));
   cudaFuncSetAttribute(ans_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(DecSmem));
-  cfg.enc_ctas = max(occupancy((const void*)ans_encode_kernel<false, false>, kEncThreads, sizeof(EncSmem)),
-                     occupancy((const void*)ans_encode_kernel<false, true>, kEncThreads, sizeof(EncSmem)));
-  cudaFuncSetAttribute(ans_encode_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(EncSmemSlots));
-  cudaFuncSetAttribute(ans_encode_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(EncSmemSlots));
-  cfg.enc_slot_ctas = max(occupancy((const void*)ans_encode_kernel<true, false>, kEncThreads,
-                                    sizeof(EncSmemSlots)),
-                          occupancy((const void*)ans_encode_kernel<true, true>, kEncThreads,
-                                    sizeof(EncSmemSlots)));
   cfg.dec_ctas = occupancy((const void*)ans_decode_kernel, kDecThreads, sizeof(DecSmem));
   cfg.hist_ctas = occupancy((const void*)hist_bytes_kernel, kHistThreads, 0);
 }
@@ -326,30 +313,32 @@ cudaError_t launch_hist_bytes(const uint8_t* in, uint64_t n, Ctrl* ctrl, int pro
 }
 
 uint64_t ans_encode_slot_bytes(const LaunchCfg& cfg) {
-  return (uint64_t)cfg.sms * cfg.enc_slot_ctas * kEncWarps * 2 * kEncSlotBytes;  // two per warp
+  return (uint64_t)cfg.sms * kEncMaxWarps * 2 * kEncSlotBytes;  // two per warp
 }
 
 cudaError_t launch_ans_encode(const uint8_t* in, uint8_t* out, uint64_t out_cap,
                               unsigned long long* out_size64, uint32_t* out_size32, Ctrl* ctrl,
-                              unsigned long long* flags, int prob_bits, uint64_t max_blocks,
-                              const LaunchCfg& cfg, cudaStream_t s, uint8_t* slots) {
-  // Both table-layout variants are launched; each decides from the pdf on
-  // the device and the one that does not match returns at once.
-  const uint64_t want = div_up_u64(max_blocks, kEncWarps);
+                              unsigned long long* flags, int prob_bits, uint64_t likely_blocks,
+                              uint64_t max_blocks, const LaunchCfg& cfg, cudaStream_t s,
+                              uint8_t* slots) {
   if (slots) {
-    const uint64_t cap = (uint64_t)cfg.sms * cfg.enc_slot_ctas;
-    const unsigned grid = (unsigned)(want < 1 ? 1 : (want < cap ? want : cap));
-    ans_encode_kernel<true, false><<<grid, kEncThreads, sizeof(EncSmemSlots), s>>>(
-        in, out, out_cap, out_size64, out_size32, ctrl, flags, prob_bits, slots);
-    ans_encode_kernel<true, true><<<grid, kEncThreads, sizeof(EncSmemSlots), s>>>(
-        in, out, out_cap, out_size64, out_size32, ctrl, flags, prob_bits, slots);
+    // one CTA per SM with as many warps as spread the blocks evenly
+    uint64_t warps = div_up_u64(likely_blocks, (uint64_t)cfg.sms);
+    warps = warps < 4 ? 4 : warps < kEncMaxWarps ? warps : kEncMaxWarps;
+    const uint64_t want = div_up_u64(max_blocks, warps);
+    const unsigned grid =
+        (unsigned)(want < 1 ? 1 : (want < (uint64_t)cfg.sms ? want : (uint64_t)cfg.sms));
+    auto* k = prob_bits == 9    ? ans_encode_slots_kernel<9>
+              : prob_bits == 10 ? ans_encode_slots_kernel<10>
+                                : ans_encode_slots_kernel<11>;
+    k<<<grid, (unsigned)warps * 32, enc_smem_bytes((int)warps), s>>>(
+        in, out, out_cap, out_size64, out_size32, ctrl, flags, slots);
   } else {
+    const uint64_t want = div_up_u64(max_blocks, kEncWarps);
     const uint64_t cap = (uint64_t)cfg.sms * cfg.enc_ctas;
     const unsigned grid = (unsigned)(want < 1 ? 1 : (want < cap ? want : cap));
-    ans_encode_kernel<false, false><<<grid, kEncThreads, sizeof(EncSmem), s>>>(
-        in, out, out_cap, out_size64, out_size32, ctrl, flags, prob_bits, nullptr);
-    ans_encode_kernel<false, true><<<grid, kEncThreads, sizeof(EncSmem), s>>>(
-        in, out, out_cap, out_size64, out_size32, ctrl, flags, prob_bits, nullptr);
+    ans_encode_shared_kernel<<<grid, kEncThreads, sizeof(EncSmem), s>>>(
+        in, out, out_cap, out_size64, out_size32, ctrl, flags, prob_bits);
   }
   return cudaGetLastError();
 }

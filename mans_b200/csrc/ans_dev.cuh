@@ -33,19 +33,8 @@ __device__ __forceinline__ EncEntry4 expand_enc_entry(uint2 e, int p) {
                    (e.y & 31u) | (cmpl << 5)};
 }
 
-struct EncSmemSlots {  // words go to global slots
-  union {
-    EncEntry4 table4[kAnsSyms];  // expanded entries
-    uint2 table2[kAnsSyms];      // packed entries
-  };
-  alignas(16) uint8_t in[kEncWarps][kEncStageBytes];
-  uint64_t bar[kEncWarps];
-};
 struct EncSmem {  // words compacted in shared memory
-  union {
-    EncEntry4 table4[kAnsSyms];
-    uint2 table2[kAnsSyms];
-  };
+  uint2 table[kAnsSyms];  // packed entries
   alignas(16) uint8_t in[kEncWarps][kEncStageBytes];
   uint64_t bar[kEncWarps];
   alignas(16) uint16_t out[kEncWarps][kEncOutWords];
@@ -67,19 +56,14 @@ template <int kP>
 __device__ __forceinline__ uint32_t enc_threshold(const uint2& e) {
   return ((1u << kP) - (e.y >> 20)) << (kAnsStateBits - kP);
 }
-template <int kP>
-__device__ __forceinline__ uint32_t enc_threshold(const EncEntry4& e) {
-  return e.thr;
-}
-
 // One interleaved step: renormalise (emit 16 bits, lanes in ascending order
 // into the compacted word buffer), then code the symbol.
 // kGuard: drop words past the buffer (see encode_words).
-template <int kP, bool kGuard, bool kShared, typename TabT>
+template <int kP, bool kGuard, bool kShared>
 __device__ __forceinline__ void enc_step(bool valid, uint32_t& x, uint32_t sym,
-                                         const TabT* __restrict__ tab, uint16_t* __restrict__ out,
+                                         const uint2* __restrict__ tab, uint16_t* __restrict__ out,
                                          uint32_t& nw, uint32_t ltmask) {
-  const TabT e = tab[sym];
+  const uint2 e = tab[sym];
   const bool wr = valid && x >= enc_threshold<kP>(e);
   const uint32_t vote = __ballot_sync(0xffffffffu, wr);
   const uint32_t idx = nw + __popc(vote & ltmask);
@@ -106,9 +90,9 @@ __device__ __forceinline__ void discard_l2_line(const void* p) {
 // The coding of one staged block (syms: the lane's first symbol in the stage,
 // bs bytes) at precision kP. kShared: sout is in shared memory (else a
 // global slot). Returns the word count; x receives the lane's final state.
-template <int kP, bool kShared, typename TabT>
+template <int kP, bool kShared>
 __device__ __forceinline__ uint32_t encode_staged(const uint8_t* syms, uint32_t bs,
-                                                  const TabT* table, uint16_t* sout, int lane,
+                                                  const uint2* table, uint16_t* sout, int lane,
                                                   uint32_t& x) {
   const uint32_t ltmask = lanemask_lt();
   x = kAnsStartState;
@@ -148,9 +132,9 @@ __device__ __forceinline__ uint32_t encode_staged(const uint8_t* syms, uint32_t 
 // interleaved coding; the word count is padded to a 16-byte multiple with
 // zeros (GpuANSEncode.h:275). Returns the number of words; x receives the
 // lane's final state.
-template <bool kSharedOut, typename TabT>
+template <bool kSharedOut>
 __device__ __forceinline__ uint32_t encode_words(const uint8_t* __restrict__ in, uint64_t n,
-                                                 uint32_t b, const TabT* table, uint8_t* stage,
+                                                 uint32_t b, const uint2* table, uint8_t* stage,
                                                  uint64_t* bar, uint32_t& parity, uint16_t* sout,
                                                  int p, const Sink& sink, int lane, uint32_t& x) {
   const uint64_t start = (uint64_t)b * kAnsBlock;
@@ -185,6 +169,158 @@ __device__ __forceinline__ uint32_t encode_words(const uint8_t* __restrict__ in,
   return nw;
 }
 
+// ---- encode with replicated tables (word slots in global memory) ----
+// The step's integer instructions bound the coder (the ALU pipe issues at half
+// rate), and shared-memory wavefronts come next. 16-byte entries need the
+// fewest instructions (24 per step, block overhead included; 29 with the
+// packed 8-byte entry) and the copies below keep a lookup at four wavefronts
+// for any distribution (unreplicated: 5 to 10 on a flat one). On 1 GiB of
+// detector frames 0.695 -> 0.641 ms, a 2 GiB uint16 volume 1.622 -> 1.321 ms,
+// 100 MB of skewed bytes 151 -> 113 us, 8 MiB of uint16 37.5 -> 21 us against
+// a table per CTA of eight warps in one of two layouts, with each step's words
+// stored to the slot in global memory.
+// Expanded entries (EncEntry4) in 8 copies: entry s of copy c at 128 s + 16 c.
+// A lane reads copy lane % 8, so the four quarter-warps of a 16-byte load
+// never conflict, whatever symbols they look up.
+constexpr uint32_t kEncTableBytes = kAnsSyms * 128;
+// A block's words collect in shared memory and leave for the slot in pieces
+// of 256 words (one 16-byte store per lane), checked every eight steps: at
+// most 255 words are left over, and eight steps add at most 256.
+constexpr uint32_t kEncPieceWords = 256;
+// Steps whose table entries are loaded ahead of the coding chain (eight spill
+// at 64 registers, and 24 warps per SM with 80 registers are slower: 0.696 ms
+// on the detector frames).
+constexpr int kEncAhead = 4;
+struct EncWarp {
+  alignas(16) uint8_t in[kEncStageBytes];
+  alignas(16) uint16_t words[2 * kEncPieceWords];
+  alignas(16) uint64_t bar;
+};
+inline size_t enc_smem_bytes(int warps) { return kEncTableBytes + (size_t)warps * sizeof(EncWarp); }
+
+// Fill the table from 256 packed entries (all threads of the CTA; the caller
+// synchronises). Rotated, so that the lanes of a store spread over the banks.
+__device__ __forceinline__ void enc_fill_table(uint8_t* tab, const uint2* __restrict__ enc, int p) {
+  for (uint32_t i = threadIdx.x; i < kAnsSyms * 8; i += blockDim.x) {
+    const uint32_t sym = i & 255u, c = (i >> 8) + sym;
+    *reinterpret_cast<EncEntry4*>(tab + 128 * sym + 16 * (c & 7)) = expand_enc_entry(enc[sym], p);
+  }
+}
+
+// One interleaved step: renormalise (16 bits of each lane whose state is at
+// its threshold, in lane order, to shared address wa on), then code. In PTX,
+// so that one predicate serves the vote, the store and the shift: the integer
+// ALU, which issues at half rate, bounds the coder.
+template <int kP>
+__device__ __forceinline__ void enc_step_rep(uint32_t& x, const EncEntry4& e, uint32_t& wa,
+                                             uint32_t ltmask) {
+  asm volatile(
+      "{\n .reg .pred p;\n .reg .b32 v, r;\n"
+      " setp.ge.u32 p, %0, %2;\n"
+      " vote.sync.ballot.b32 v, p, 0xffffffff;\n"
+      " and.b32 r, v, %3;\n popc.b32 r, r;\n mad.lo.u32 r, r, 2, %1;\n"
+      " @p st.shared.u16 [r], %0;\n"
+      " popc.b32 v, v;\n mad.lo.u32 %1, v, 2, %1;\n"
+      " @p shr.u32 %0, %0, 16;\n}\n"
+      : "+r"(x), "+r"(wa) : "r"(e.thr), "r"(ltmask) : "memory");
+  x = enc_code<kP>(x, e);
+}
+// The same for a partial step: only lanes with `valid` hold a symbol.
+template <int kP>
+__device__ __forceinline__ void enc_step_part(bool valid, uint32_t& x, const EncEntry4& e,
+                                              uint32_t& wa,
+                                              uint32_t ltmask) {
+  const bool wr = valid && x >= e.thr;
+  const uint32_t vote = __ballot_sync(0xffffffffu, wr);
+  if (wr) {
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(wa + 2u * __popc(vote & ltmask)), "r"(x) : "memory");
+    x >>= 16;
+  }
+  wa += 2u * __popc(vote);
+  if (valid) x = enc_code<kP>(x, e);
+}
+
+// Encode a staged block (syms: the lane's first symbol in the stage, bs bytes)
+// into its word slot, padded to a multiple of eight words with zeros. Returns
+// the word count; x receives the lane's final state.
+template <int kP>
+__device__ __forceinline__ uint32_t encode_staged_rep(const uint8_t* syms, uint32_t bs,
+                                                      const uint8_t* tab, uint16_t* words,
+                                                      uint8_t* slot, int lane, uint32_t& x) {
+  const uint32_t ltmask = lanemask_lt();
+  const uint32_t wb = smem_addr(words);
+  const uint8_t* const tl = tab + 16 * (lane & 7);
+  auto entry = [&](uint32_t sym) { return *reinterpret_cast<const EncEntry4*>(tl + 128 * sym); };
+  x = kAnsStartState;
+  uint32_t wa = wb, done = 0;  // shared address of the next word; bytes in the slot
+  const uint32_t full = bs >> 5;
+  uint32_t j = 0;
+#pragma unroll 1
+  for (; j + 8 <= full; j += 8) {
+#pragma unroll
+    for (int h = 0; h < 8; h += kEncAhead) {
+      EncEntry4 e[kEncAhead];
+#pragma unroll
+      for (int u = 0; u < kEncAhead; ++u) e[u] = entry(syms[(j + h + u) * 32]);
+#pragma unroll
+      for (int u = 0; u < kEncAhead; ++u) enc_step_rep<kP>(x, e[u], wa, ltmask);
+    }
+    if (wa - wb >= 2 * kEncPieceWords) {
+      __syncwarp();
+      const uint4* src = reinterpret_cast<const uint4*>(words) + lane;
+      const uint4 v = src[0], r = src[32];
+      // a slot holds any block whose words fit the bound; more only come from
+      // a table that does not belong to the bytes, and are dropped
+      if (done + 2 * kEncPieceWords <= kEncSlotBytes)
+        *reinterpret_cast<uint4*>(slot + done + 16 * lane) = v;
+      __syncwarp();
+      reinterpret_cast<uint4*>(words)[lane] = r;
+      __syncwarp();
+      wa -= 2 * kEncPieceWords;
+      done += 2 * kEncPieceWords;
+    }
+  }
+  for (; j < full; ++j) enc_step_rep<kP>(x, entry(syms[j * 32]), wa, ltmask);
+  if (bs & 31) {
+    const bool valid = (uint32_t)lane < (bs & 31);
+    enc_step_part<kP>(valid, x, entry(valid ? syms[j * 32] : 0u), wa, ltmask);
+  }
+  const uint32_t rem = (wa - wb) >> 1;  // < 512
+  const uint32_t padded = (rem + 7) & ~7u;
+  __syncwarp();
+  if ((uint32_t)lane < padded - rem) words[rem + lane] = 0;
+  __syncwarp();
+  for (uint32_t i = lane; i < padded / 8; i += 32)
+    if (done + 16 * i + 16 <= kEncSlotBytes)
+      *reinterpret_cast<uint4*>(slot + done + 16 * i) = reinterpret_cast<const uint4*>(words)[i];
+  return done / 2 + rem;
+}
+
+// encode_words for the replicated table: block b of one buffer (one warp).
+template <int kP>
+__device__ __forceinline__ uint32_t encode_words_rep(const uint8_t* __restrict__ in, uint64_t n,
+                                                     uint32_t b, const uint8_t* tab, EncWarp& sw,
+                                                     uint32_t& parity, uint16_t* slot,
+                                                     const Sink& sink, int lane, uint32_t& x) {
+  const uint64_t start = (uint64_t)b * kAnsBlock;
+  const uint32_t bs = (uint32_t)min_u64(kAnsBlock, n - start);
+  __syncwarp();  // the previous block's reads of the stage are complete
+  if (lane == 0) {
+    const uintptr_t a0 = reinterpret_cast<uintptr_t>(in + start) & ~uintptr_t(15);
+    const uintptr_t a1 = (reinterpret_cast<uintptr_t>(in + start) + bs + 15) & ~uintptr_t(15);
+    bulk_load(sw.in, reinterpret_cast<const void*>(a0), (uint32_t)(a1 - a0), &sw.bar);
+  }
+  if (!mbar_wait(&sw.bar, parity) && lane == 0) report(sink, MANS_ERR_TIMEOUT, b);
+  parity ^= 1u;
+  uint32_t nw = encode_staged_rep<kP>(sw.in + phase16(in + start) + lane, bs, tab, sw.words,
+                                      reinterpret_cast<uint8_t*>(slot), lane, x);
+  if (nw > kAnsMaxBlockWords) {  // see encode_words
+    if (lane == 0) report(sink, MANS_ERR_CORRUPT, b);
+    nw = kAnsMaxBlockWords;
+  }
+  return nw;
+}
+
 // Store block b, whose nw words (padded to padded) start at word `prefix` of
 // the stream's data section: lane states, block word entry, the words, and
 // for the buffer's last block the header, pdf and size. Then the slot's
@@ -210,9 +346,19 @@ __device__ __forceinline__ void encode_store(uint8_t* __restrict__ out, uint64_t
     if (lane == 0) bw[b] = make_uint2((bs << 16) | nw, prefix);
     uint4* dst = reinterpret_cast<uint4*>(out + over + 2ull * prefix);
     const uint4* src = reinterpret_cast<const uint4*>(sout);
-    for (uint32_t i = lane; i < padded / 8; i += 32) {
-      if (kSlots) dst[i] = __ldcg(src + i);
-      else dst[i] = src[i];
+    const uint32_t cnt = padded / 8;
+    if (kSlots) {  // four loads in flight per lane
+      for (uint32_t i = lane; i < cnt; i += 128) {
+        uint4 v[4];
+#pragma unroll
+        for (uint32_t h = 0; h < 4; ++h)
+          if (i + 32 * h < cnt) v[h] = __ldcg(src + i + 32 * h);
+#pragma unroll
+        for (uint32_t h = 0; h < 4; ++h)
+          if (i + 32 * h < cnt) dst[i + 32 * h] = v[h];
+      }
+    } else {
+      for (uint32_t i = lane; i < cnt; i += 32) dst[i] = src[i];
     }
     if (last) {
       if (lane < 8) {
@@ -271,11 +417,11 @@ __device__ __forceinline__ void encode_finish(
 
 // One block as the unit of the single-pass prefix (flags per block): encode,
 // publish the aggregate, look back, store.
-template <bool kSlots, typename TabT>
+template <bool kSlots>
 __device__ __forceinline__ void encode_block(
     const uint8_t* __restrict__ in, uint64_t n, uint8_t* __restrict__ out, uint64_t out_cap,
     unsigned long long* out_size64, uint32_t* out_size32, const uint32_t* __restrict__ pdf,
-    unsigned long long* flags, uint32_t epoch, int p, const Sink& sink, const TabT* table,
+    unsigned long long* flags, uint32_t epoch, int p, const Sink& sink, const uint2* table,
     uint8_t* stage, uint64_t* bar, uint32_t& parity, uint16_t* sout, uint32_t b, int lane) {
   uint32_t x;
   const uint32_t nw =

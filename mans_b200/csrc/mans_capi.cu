@@ -191,7 +191,7 @@ mans_status compress_impl(mans_workspace* ws, mans_dtype dtype, mans_layout layo
     mark(ws, 1, s);
     if (e == cudaSuccess)
       e = launch_ans_encode((const uint8_t*)d_in, (uint8_t*)d_out, out_capacity, osz, nullptr,
-                            ws->ctrl, ws->ans_flags, precision,
+                            ws->ctrl, ws->ans_flags, precision, div_up_u64(in_bytes, kAnsBlock),
                             div_up_u64(in_bytes, kAnsBlock), ws->cfg, s, ws->enc_slots);
     mark(ws, 2, s);
     return e == cudaSuccess ? MANS_OK : MANS_ERR_CUDA;
@@ -217,9 +217,10 @@ mans_status compress_impl(mans_workspace* ws, mans_dtype dtype, mans_layout layo
           m, (uint8_t*)d_out, out_capacity, ws->ctrl, osz);
       e = cudaGetLastError();
     } else {
+      // an element maps to one byte, and a little more
       e = launch_ans_encode(m, (uint8_t*)d_out, out_capacity, osz, nullptr, ws->ctrl,
-                            ws->ans_flags, precision, div_up_u64(ws->merged_cap, kAnsBlock),
-                            ws->cfg, s, ws->enc_slots);
+                            ws->ans_flags, precision, div_up_u64(n_elems + n_elems / 4, kAnsBlock),
+                            div_up_u64(ws->merged_cap, kAnsBlock), ws->cfg, s, ws->enc_slots);
     }
   }
   mark(ws, 2, s);
@@ -551,7 +552,7 @@ mans_status mans_ans_encode(int precision, const uint8_t* d_in, uint32_t in_size
   if (e == cudaSuccess)
     e = launch_ans_encode(d_in, d_out, ans_bound(in_size), nullptr, d_out_size, ws->ctrl,
                           ws->ans_flags, precision, div_up_u64(in_size, kAnsBlock),
-                          ws->cfg, s, ws->enc_slots);
+                          div_up_u64(in_size, kAnsBlock), ws->cfg, s, ws->enc_slots);
   return e == cudaSuccess ? MANS_OK : MANS_ERR_CUDA;
 }
 

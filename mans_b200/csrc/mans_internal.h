@@ -23,7 +23,6 @@ struct NvtxRange {
 struct LaunchCfg {
   int sms = 148;        // multiprocessors of the device
   int enc_ctas = 0;     // resident CTAs per SM of the encode kernel (shared-memory staging)
-  int enc_slot_ctas = 0;  // resident CTAs per SM of the encode kernel (global slots)
   int dec_ctas = 0;     // resident CTAs per SM of the decode kernel
   int map_ctas = 0;     // resident CTAs per SM of the ADM map kernels
   int map32_ctas = 0;   // resident CTAs per SM of the uint32 ADM map kernel
@@ -39,13 +38,15 @@ void init_launch_cfg(LaunchCfg& cfg, int device);
 cudaError_t launch_hist_bytes(const uint8_t* in, uint64_t n, Ctrl* ctrl, int prob_bits,
                               const LaunchCfg& cfg, cudaStream_t s);
 // Encode ctrl->merged_size bytes at `in` (table from ctrl) into the coalesced
-// stream at `out`. max_blocks bounds the number of 4 KiB blocks (grid size).
+// stream at `out`. max_blocks bounds the number of 4 KiB blocks (grid size);
+// likely_blocks is what is to be expected (warps per CTA).
 // slots: ans_encode_slot_bytes(cfg) bytes of global scratch for the words of
 // blocks in flight, or nullptr to compact them in shared memory instead.
 cudaError_t launch_ans_encode(const uint8_t* in, uint8_t* out, uint64_t out_cap,
                               unsigned long long* out_size64, uint32_t* out_size32, Ctrl* ctrl,
-                              unsigned long long* flags, int prob_bits, uint64_t max_blocks,
-                              const LaunchCfg& cfg, cudaStream_t s, uint8_t* slots);
+                              unsigned long long* flags, int prob_bits, uint64_t likely_blocks,
+                              uint64_t max_blocks, const LaunchCfg& cfg, cudaStream_t s,
+                              uint8_t* slots);
 uint64_t ans_encode_slot_bytes(const LaunchCfg& cfg);
 // Decode the stream at `in` into `out` (at most out_cap bytes). expect_p < 0
 // accepts any valid precision. record != 0 stores the decoded size in ctrl.
