@@ -211,7 +211,7 @@ __device__ __forceinline__ void map32_group(const uint32_t* __restrict__ in, uin
     atomicAdd(&hist[c >> 24], 1u);
   }
   __syncwarp();
-  // store: M + rec_base is 16-byte aligned and goff a multiple of 8
+  // store: M is 16-byte aligned, rec_base and goff multiples of 8
   if (rec_base + (uint64_t)goff + gtot <= m_cap) {
     uint2* dst = reinterpret_cast<uint2*>(M + rec_base + goff);
     const uint2* src = reinterpret_cast<const uint2*>(stage);

@@ -195,43 +195,104 @@ __global__ __launch_bounds__(kEncThreads) void ans_encode_shared_kernel(
 }
 
 // ------------------------------------------------------------------------
-// Decode: one warp per block, decoded from its last step to its first. The
-// block's words are staged in shared memory with one bulk copy (read
-// backwards, data-dependently, every step); decoded bytes collect in a
-// 512-byte per-warp stage and leave as 16-byte stores every 16 steps. The
-// next block is claimed early and its words prefetched into L2 (no
-// look-back: claiming ahead costs nothing here).
+// Decode: a warp decodes a block, or two together, from the last step to the
+// first. One CTA of up to 32 warps per SM shares the replicated slot table
+// (128 KiB). What bounds it: per step 21 instructions of which 7 go to the
+// half-rate integer ALU, two population counts, and a chain of two
+// shared-memory loads, a vote and a population count (about 130 cycles) that
+// only other chains can hide. The former kernel (22 instructions, 12 of them
+// ALU, table conflicts on 40% of its shared wavefronts, 32 chains per SM
+// instead of 64) took 0.575 ms on 1 GiB of detector frames (here 0.525), 1.092
+// on a 2 GiB uint16 volume (1.042), 27.7 us on 8 MiB of uint16 (21.0) and 131 us
+// on 100 MB of skewed bytes at p = 11 (105; its drop-in call also launched half
+// a resident wave). A single block takes 14.4 us instead of 13.4.
 // ------------------------------------------------------------------------
-struct DecSmem {
-  uint32_t lut[1 << kMaxProbBits];  // below every warp's stage (see decode_full_smem)
-  DecWarpSmem warp[kDecWarps];
-  uint64_t bar[kDecWarps];
-};
-// Four CTAs of eight warps per SM (32 warps): 50 KiB of shared memory each,
-// with word stages of 2,560 words, so that blocks of poorly compressible
-// bytes (about 2,048 words) also decode from shared memory (5 CTAs with
-// 2,048-word stages: 1 GiB of gradient data decoded in 1.30 ms, here 0.59).
-constexpr int kDecMinCtas = 4;
+constexpr int kDecMaxWarps = 32, kDecMinWarps = 8;
+constexpr size_t kDecStageMax = (size_t)kDecMaxWarps * 2 * sizeof(DecWarp);
+constexpr size_t dec_stage_bytes(size_t warps, int blocks) {
+  return warps * sizeof(DecWhole) <= kDecStageMax ? warps * sizeof(DecWhole)
+                                                  : warps * blocks * sizeof(DecWarp);
+}
 
-__global__ __launch_bounds__(kDecThreads, kDecMinCtas) void ans_decode_kernel(
+// kBlocks: blocks that a warp takes at a time and decodes together (one at a
+// time once less than a block per warp of the grid is left, so that the last
+// wave is short). Each warp's first blocks are fixed, spread over the CTAs, and
+// the rest is claimed: a small input then takes no claim at all (4,736 warps on
+// one counter cost 5 us). The next claim and its prefetches come in the middle
+// of the current blocks, where other warps hide their latency.
+template <int kP, int kBlocks>
+__device__ __forceinline__ void decode_blocks(const uint8_t* __restrict__ in, uint32_t nb, uint32_t n,
+                                              uint32_t cw, uint8_t* __restrict__ out,
+                                              const uint8_t* lut, uint8_t* stage, uint32_t stage_bytes,
+                                              Ctrl* ctrl, const Sink& sink, int lane) {
+  auto bad = [&](uint32_t k) { report(sink, MANS_ERR_CORRUPT, k); };
+  const uint32_t warp = threadIdx.x >> 5;
+  if ((uint64_t)stage_bytes / sizeof(DecWhole) * gridDim.x >= nb) {
+    // a block per warp at most, and room to stage its words whole
+    const uint32_t k = warp * gridDim.x + blockIdx.x;
+    if (k < nb)
+      decode_block<kP, 1>(in, nb, n, cw, out, lut, reinterpret_cast<DecWhole*>(stage) + warp, k, lane,
+                          [](int) {}, bad);
+    return;
+  }
+  DecWarp* const ws = reinterpret_cast<DecWarp*>(stage) + kBlocks * warp;
+  const uint8_t* states = in + kAnsHeaderBytes + 2 * kAnsSyms;
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  const uint32_t first = kBlocks == 2 && nb > warps ? 2u : 1u;  // blocks per warp at the start
+  auto claim = [&](uint32_t seen, uint32_t& take) {
+    take = kBlocks == 2 && seen < nb && nb - seen > warps ? 2u : 1u;
+    if (first * warps >= nb) return nb;
+    uint32_t v = 0;
+    if (lane == 0) v = first * warps + atomicAdd(&ctrl->tile_counter[2], take);
+    return __shfl_sync(0xffffffffu, v, 0);
+  };
+  uint32_t take = first;
+  uint32_t b = first * (warp * gridDim.x + blockIdx.x);
+  while (b < nb) {
+    uint32_t nxt = 0, nxt_take = 0;
+    auto hook = [&](int c) {
+      if (c != 3) return;
+      nxt = claim(b, nxt_take);
+      if (lane < kBlocks && lane < nxt_take && nxt + lane < nb) {
+        const uint2 bn = __ldg(reinterpret_cast<const uint2*>(states + 128ull * nb) + nxt + lane);
+        prefetch_l2(states + 128ull * (nxt + lane), 128);
+        const uint32_t wn = ((bn.x & 0xffffu) + 7) & ~7u;
+        if ((uint64_t)bn.y + wn <= cw) prefetch_l2(in + ans_overhead(nb) + 2ull * bn.y, 2 * wn);
+      }
+    };
+    if (kBlocks == 2 && take == 2 && b + 2 < nb) {
+      decode_block<kP, kBlocks>(in, nb, n, cw, out, lut, ws, b, lane, hook, bad);
+    } else {
+      // one by one; the last block may be short (and has no fixed chunks)
+      for (uint32_t k = b; k < nb && k < b + take; ++k)
+        decode_block<kP, 1>(in, nb, n, cw, out, lut, ws, k, lane, [](int) {}, bad);
+      nxt = claim(b, nxt_take);
+    }
+    b = nxt;
+    take = nxt_take;
+  }
+}
+
+template <int kBlocks>
+__global__ __launch_bounds__(kDecMaxWarps * 32, 1) void ans_decode_kernel(
     const uint8_t* __restrict__ in, uint64_t in_size, uint8_t* __restrict__ out, uint64_t out_cap,
-    Ctrl* ctrl, int expect_p, int record) {
+    Ctrl* ctrl, int expect_p, int record, uint32_t stage_bytes) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
-  DecSmem& sm = *reinterpret_cast<DecSmem*>(smem_raw);
-  __shared__ uint32_t s_scan[kDecWarps];
-  __shared__ int s_ok, s_last;
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  uint64_t* bar = &sm.bar[warp];
-  if (lane == 0) mbar_init(bar);
-  uint32_t parity = 0;
+  __shared__ uint32_t s_incl[kAnsSyms];
+  __shared__ int s_ok;
+  const int t = threadIdx.x, lane = t & 31;
+  uint8_t* const lut = smem_raw;  // below every warp's words (see decode_block)
+  uint8_t* const stage = smem_raw + kDecLutBytes;
   const Sink sink = sink_of(ctrl);
 
   // ---- header validation (GpuANSCodec.h:106-113 asserts, GpuANSDecode.h:220-227)
   uint32_t h[5] = {0, 0, 0, 0, 0};
+  uint32_t pdf = 0;
   bool ok = in_size >= kAnsHeaderBytes + 2 * kAnsSyms;
   if (ok) {
 #pragma unroll
     for (int i = 0; i < 5; ++i) h[i] = __ldg(reinterpret_cast<const uint32_t*>(in) + i);
+    pdf = dec_pdf(in);
   }
   const uint32_t nb = h[1], n = h[2], cw = h[3];
   const int p = (int)(h[4] & 0xfu);
@@ -244,40 +305,26 @@ __global__ __launch_bounds__(kDecThreads, kDecMinCtas) void ans_decode_kernel(
   if (record && ok && blockIdx.x == 0 && t == 0) ctrl->merged_size = n;
   __syncthreads();
 
-  if (s_ok && n > 0) {
-    const bool tables_ok = build_decode_tables(in, p, sm.lut, s_scan);
-    if (!tables_ok && t == 0) {
-      s_ok = 0;
-      if (blockIdx.x == 0) report(sink, MANS_ERR_BAD_STREAM, 1);
-    }
-  }
-  __syncthreads();
-
-  if (s_ok && n > 0) {
-    const uint64_t over = ans_overhead(nb);
-    const uint2* bwords = reinterpret_cast<const uint2*>(in + kAnsHeaderBytes + 2 * kAnsSyms + 128ull * nb);
-    uint32_t b = warp_claim(&ctrl->tile_counter[2], lane);
-    while (b < nb) {
-      const uint32_t nxt = warp_claim(&ctrl->tile_counter[2], lane);
-      if (nxt < nb && lane == 0) {
-        const uint2 bn = __ldg(bwords + nxt);
-        const uint32_t wn = ((bn.x & 0xffffu) + 7) & ~7u;
-        if ((uint64_t)bn.y + wn <= cw) prefetch_l2(in + over + 2ull * bn.y, 2 * wn);
+  if (s_ok && blockIdx.x < nb) {  // CTA k holds block k at least
+    const bool tables_ok = dec_build_lut(pdf, p, lut, s_incl);
+    if (!tables_ok && blockIdx.x == 0 && t == 0) report(sink, MANS_ERR_BAD_STREAM, 1);
+    __syncthreads();
+    if (tables_ok) {
+      switch (p) {
+        case 9: decode_blocks<9, kBlocks>(in, nb, n, cw, out, lut, stage, stage_bytes, ctrl, sink, lane); break;
+        case 10: decode_blocks<10, kBlocks>(in, nb, n, cw, out, lut, stage, stage_bytes, ctrl, sink, lane); break;
+        default: decode_blocks<11, kBlocks>(in, nb, n, cw, out, lut, stage, stage_bytes, ctrl, sink, lane); break;
       }
-      decode_block(in, nb, n, cw, p, out, sm.lut, &sm.warp[warp], bar, parity, sink, b, lane);
-      b = nxt;
     }
   }
 
   __syncthreads();
   if (t == 0) {
     __threadfence();
-    s_last = atomicAdd(&ctrl->done_counter[2], 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (s_last && t == 0) {
-    ctrl->tile_counter[2] = 0;
-    ctrl->done_counter[2] = 0;
+    if (atomicAdd(&ctrl->done_counter[2], 1u) == gridDim.x - 1) {
+      ctrl->tile_counter[2] = 0;
+      ctrl->done_counter[2] = 0;
+    }
   }
 }
 
@@ -297,9 +344,10 @@ void init_ans_launch_cfg(LaunchCfg& cfg) {
   cudaFuncSetAttribute(ans_encode_shared_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(EncSmem));
   cfg.enc_ctas = occupancy((const void*)ans_encode_shared_kernel, kEncThreads, sizeof(EncSmem));
-  cudaFuncSetAttribute(ans_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(DecSmem));
-  cfg.dec_ctas = occupancy((const void*)ans_decode_kernel, kDecThreads, sizeof(DecSmem));
+  cudaFuncSetAttribute(ans_decode_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)(kDecLutBytes + kDecStageMax));
+  cudaFuncSetAttribute(ans_decode_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)(kDecLutBytes + kDecStageMax));
   cfg.hist_ctas = occupancy((const void*)hist_bytes_kernel, kHistThreads, 0);
 }
 
@@ -344,13 +392,22 @@ cudaError_t launch_ans_encode(const uint8_t* in, uint8_t* out, uint64_t out_cap,
 }
 
 cudaError_t launch_ans_decode(const uint8_t* in, uint64_t in_size, uint8_t* out, uint64_t out_cap,
-                              Ctrl* ctrl, int expect_p, int record, uint64_t max_blocks,
-                              const LaunchCfg& cfg, cudaStream_t s) {
-  uint64_t want = div_up_u64(max_blocks, kDecWarps);
-  uint64_t cap = (uint64_t)cfg.sms * cfg.dec_ctas;
-  unsigned grid = (unsigned)(want < 1 ? 1 : (want < cap ? want : cap));
-  ans_decode_kernel<<<grid, kDecThreads, sizeof(DecSmem), s>>>(in, in_size, out, out_cap, ctrl,
-                                                                expect_p, record);
+                              Ctrl* ctrl, int expect_p, int record, uint64_t likely_blocks,
+                              uint64_t max_blocks, const LaunchCfg& cfg, cudaStream_t s) {
+  // One CTA per SM with as many warps as spread the blocks evenly; a warp takes
+  // two blocks together once a block per warp does not hold them all (16 M
+  // uint16 values, 30 blocks per SM: decode 31 us one by one, 36 in pairs; 24 M,
+  // 45 per SM: 50 and 40; 1 GiB of detector frames: 0.591 and 0.525 ms).
+  const int blocks = likely_blocks > (uint64_t)cfg.sms * kDecMaxWarps ? 2 : 1;
+  uint64_t warps = div_up_u64(likely_blocks, (uint64_t)cfg.sms * blocks);
+  warps = warps < kDecMinWarps ? kDecMinWarps : warps < kDecMaxWarps ? warps : kDecMaxWarps;
+  const uint64_t want = div_up_u64(max_blocks, warps * blocks);
+  const unsigned grid =
+      (unsigned)(want < 1 ? 1 : (want < (uint64_t)cfg.sms ? want : (uint64_t)cfg.sms));
+  auto* k = blocks == 2 ? ans_decode_kernel<2> : ans_decode_kernel<1>;
+  const size_t stage = dec_stage_bytes(warps, blocks);
+  k<<<grid, (unsigned)warps * 32, kDecLutBytes + stage, s>>>(in, in_size, out, out_cap, ctrl, expect_p,
+                                                             record, (uint32_t)stage);
   return cudaGetLastError();
 }
 

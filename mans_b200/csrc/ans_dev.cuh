@@ -432,66 +432,108 @@ __device__ __forceinline__ void encode_block(
                         EncPending{b, nw, x, sout}, lane);
 }
 
-constexpr int kDecWarps = 8;
-constexpr int kDecThreads = kDecWarps * 32;
+// ---- decode ----
 constexpr int kMaxProbBits = 11;
 
-// Build the slot table of a stream's pdf in shared memory (one CTA of 256
-// threads, thread t owns symbol t): lut[s] = pdf << 20 | (s - cdf) << 8 |
-// symbol (GpuANSDecode.h:307-377 packs the same fields in one word, in
-// another order). Returns false when the pdf does not sum to 2^p.
-__device__ __forceinline__ bool build_decode_tables(const uint8_t* __restrict__ in, int p,
-                                                    uint32_t* lut, uint32_t* s_scan) {
+// The slot table of a stream's pdf, 8 bytes per slot s of symbol y:
+//   {P = pdf << (32 - p), D << 8 | y}, D = (s - cdf) - (s * pdf >> p) (signed),
+// so that the decoder's new state pdf * (x >> p) + (s - cdf), s = x mod 2^p
+// (GpuANSDecode.h:307-377), is umulhi(x, P) + D: umulhi(x, P) = x * pdf >> p =
+// pdf * (x >> p) + (s * pdf >> p), exactly, and the second term depends on s
+// alone. (pdf = 2^p, a single symbol: P = 2^32 - 1 and D = 1, since the state
+// x >= 1 stays as it is.)
+// The table is kept in 16 copies (p <= 10) or 8 (p = 11): with n copies, copy c
+// of slot s at byte 8 (n s + c). Slots are uniformly distributed whatever the data, so
+// with one copy the 32 lookups of a step take about 6 shared-memory
+// wavefronts; a lane that reads its own copy (lane modulo the copies) takes 2
+// (16 copies) or 4 (8).
+constexpr uint32_t kDecLutBytes = 128u << 10;
+__host__ __device__ constexpr int dec_copy_bits(int p) { return p <= 10 ? 4 : 3; }
+__device__ __forceinline__ uint2 make_dec_entry(uint32_t pdf, uint32_t s, uint32_t cdf, uint32_t sym,
+                                                int p) {
+  if (pdf >> p) return make_uint2(0xffffffffu, (1u << 8) | sym);
+  return make_uint2(pdf << (32 - p), ((s - cdf - ((s * pdf) >> p)) << 8) | sym);
+}
+
+// Build the table (all threads of a CTA of at least 256; pdf: symbol
+// threadIdx.x's, dec_pdf; s_incl: 256 words of shared scratch). Each slot finds its symbol by bisection of the inclusive
+// prefix sums, so a concentrated pdf costs no more than a flat one. Returns
+// false, in every thread, when the pdf does not sum to 2^p. The caller
+// synchronises before the table is read.
+__device__ __forceinline__ uint32_t dec_pdf(const uint8_t* __restrict__ in) {
+  return threadIdx.x < kAnsSyms
+             ? __ldg(reinterpret_cast<const uint16_t*>(in + kAnsHeaderBytes) + threadIdx.x)
+             : 0u;
+}
+__device__ __forceinline__ bool dec_build_lut(uint32_t pdf, int p, uint8_t* lut,
+                                              uint32_t* s_incl) {
+  __shared__ uint32_t s_sum[8];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const uint16_t* probs = reinterpret_cast<const uint16_t*>(in + kAnsHeaderBytes);
-  const uint32_t pdf = __ldg(probs + t);
   uint32_t incl = pdf;
+  __syncthreads();  // earlier readers of the table and the scratch are done
+  if (t < kAnsSyms) {
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) s_sum[warp] = incl;
   }
-  __syncthreads();
-  if (lane == 31) s_scan[warp] = incl;
   __syncthreads();
   uint32_t base = 0, total = 0;
-  for (int w = 0; w < kDecWarps; ++w) {
-    if (w < warp) base += s_scan[w];
-    total += s_scan[w];
+#pragma unroll
+  for (int w = 0; w < 8; ++w) {
+    if (w < warp) base += s_sum[w];
+    total += s_sum[w];
   }
-  const uint32_t cdf = base + incl - pdf;
+  if (t < kAnsSyms) s_incl[t] = base + incl;
+  __syncthreads();
   if (total != (1u << p)) return false;
-  for (uint32_t j = 0; j < pdf; ++j) {
-    lut[cdf + j] = (pdf << 20) | (j << 8) | (uint32_t)t;
+#pragma unroll 4
+  for (uint32_t s = t; s < (1u << p); s += blockDim.x) {
+    uint32_t sym = 0;  // the first symbol whose inclusive sum exceeds s
+#pragma unroll
+    for (uint32_t h = 128; h > 0; h >>= 1)
+      if (s_incl[sym + h - 1] <= s) sym += h;
+    const uint32_t hi = s_incl[sym], lo = sym ? s_incl[sym - 1] : 0u;
+    const uint2 e = make_dec_entry(hi - lo, s, lo, sym, p);
+    // a row of copies, rotated so that the lanes of a store spread over the banks
+    const uint32_t n16 = 1u << (dec_copy_bits(p) - 1);
+    uint4* row = reinterpret_cast<uint4*>(lut) + s * n16;
+    for (uint32_t c = 0; c < n16; ++c) row[(c + lane) & (n16 - 1)] = make_uint4(e.x, e.y, e.x, e.y);
   }
   return true;
 }
 
-// ---- decode ----
-// Words staged in shared memory per warp (5 KiB): every block whose padded
-// word count fits -- all blocks but those of bytes that the coding expands by
-// a quarter or more -- decodes from shared memory; a block with more words
-// reads its words from global memory instead.
-constexpr uint32_t kDecStageWords = 2560;
+// A block's words are read backwards through a window of two pieces of 256
+// words: eight steps read at most one piece, so it is checked every eight
+// steps whether the lower piece has been entered, which then moves up, while
+// the piece below it, loaded a move ahead, takes its place.
+constexpr uint32_t kDecPieceWords = 256;
 // Decoded bytes leave through a per-warp 512-byte stage, 16 steps at a time,
 // as one 16-byte store per lane.
 constexpr int kDecChunkSteps = 16;
 constexpr uint32_t kDecChunkBytes = kDecChunkSteps * 32;
 
-struct DecWarpSmem {
-  alignas(16) uint16_t words[kDecStageWords];
+struct DecWarp {
+  static constexpr bool kWhole = false;
+  alignas(16) uint16_t words[2 * kDecPieceWords];
   alignas(16) uint8_t out[kDecChunkBytes + 16];  // a chunk at its destination's phase
 };
+// Where few warps share the shared memory, a block's words are staged whole,
+// without the window's moves and checks.
+struct DecWhole {
+  static constexpr bool kWhole = true;
+  alignas(16) uint16_t words[kEncOutWords];
+  alignas(16) uint8_t out[kDecChunkBytes + 16];
+};
 
-__device__ __forceinline__ uint32_t ld_shared_u16(uint32_t addr) {
-  uint16_t v;
-  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
-  return v;
+// ---- asynchronous 16-byte copies global -> shared ----
+__device__ __forceinline__ void cp_async16(uint32_t smem, const void* g) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(g) : "memory");
 }
-__device__ __forceinline__ uint32_t ld_shared_u32(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
-  return v;
+__device__ __forceinline__ void cp_async_wait_all() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 // Store one decoded 512-byte chunk from the warp's stage, where it sits at
@@ -512,118 +554,203 @@ __device__ __forceinline__ void dec_flush_chunk(uint8_t* __restrict__ g, const u
   }
 }
 
-// The 128 steps of a full block whose words are staged in shared memory, for
-// precision kP. State x per lane; wa: shared byte address one past the next
-// word to read (words are read backwards, the highest reading lane first,
-// GpuANSDecode.h:78-92); lut: shared address of the slot table. Each step:
-// slot -> table entry {pdf:12, slot - cdf:12, symbol:8}; x = pdf * (x >> p) +
-// (slot - cdf); lanes whose state fell below 2^15 read one word each.
-// A corrupt stream can move wa below the warp's words, by at most 128 steps x
-// 32 words = 8 KiB; the slot table (8 KiB) lies below every warp's words in
-// the CTA's shared memory, so such reads stay inside it, and the final
-// position check reports the block. Returns false when the block does not
-// end exactly at its first word in the start state.
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_shared_v4(uint32_t a, const uint4& v) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z),
+               "r"(v.w) : "memory");
+}
+
+// The window over a block's words.
+struct DecWindow {
+  const uint4* below;  // this lane's unit (16 bytes) of the piece below the window
+  uint4 next;          // ... loaded
+  uint32_t base;       // pieces below the window
+  uint32_t wb, wa;     // shared addresses: the window, one past the next word to read
+
+  // Load `next` where want holds. A predicated load in straight-line code: on a
+  // branch of its own, the merge with the old value would wait for the load.
+  __device__ __forceinline__ void fetch(bool want) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.u32 p, %5, 0;\n"
+        " @p ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];\n}\n"
+        : "+r"(next.x), "+r"(next.y), "+r"(next.z), "+r"(next.w)
+        : "l"(below), "r"((uint32_t)want));
+  }
+  // The caller synchronises the warp before (the memory's previous readers)
+  // and after.
+  __device__ __forceinline__ void open(const uint16_t* data, uint32_t nw, uint16_t* w, int lane) {
+    const uint4* g = reinterpret_cast<const uint4*>(data);
+    const uint32_t total = (nw + 7) / 8;  // units of the block
+    base = nw > 2 * kDecPieceWords ? (nw - 1) / kDecPieceWords - 1 : 0u;
+    wb = smem_addr(w);
+    wa = wb + 2 * (nw - base * kDecPieceWords);
+    next = make_uint4(0, 0, 0, 0);
+    const uint32_t lo = base * (kDecPieceWords / 8) + lane;
+    below = g + lo - (kDecPieceWords / 8);
+    fetch(base != 0);
+    // past L1, of which the table and the windows leave little
+    if (lo < total) cp_async16(wb + 16 * lane, g + lo);
+    if (lo + kDecPieceWords / 8 < total)
+      cp_async16(wb + 2 * kDecPieceWords + 16 * lane, g + lo + kDecPieceWords / 8);
+    cp_async_wait_all();
+  }
+  __device__ __forceinline__ void open_whole(const uint16_t* data, uint32_t nw, uint16_t* w,
+                                             int lane) {
+    base = 0;
+    wb = smem_addr(w);
+    wa = wb + 2 * nw;
+    for (uint32_t i = lane; i < (nw + 7) / 8; i += 32)
+      cp_async16(wb + 16 * i, reinterpret_cast<const uint4*>(data) + i);
+    cp_async_wait_all();
+  }
+  // Before at most eight steps.
+  __device__ __forceinline__ void advance(int lane) {
+    const bool move = base != 0 && wa - wb < 2 * kDecPieceWords;
+    if (move) {
+      __syncwarp();
+      // each unit is read and written by one lane
+      st_shared_v4(wb + 2 * kDecPieceWords + 16 * lane, ld_shared_v4(wb + 16 * lane));
+      st_shared_v4(wb + 16 * lane, next);
+      __syncwarp();
+      wa += 2 * kDecPieceWords;
+      --base;
+      below -= kDecPieceWords / 8;
+    }
+    fetch(move && base != 0);
+  }
+};
+
+// Renormalise: lanes whose state fell below 2^15 read one word each, the
+// highest reading lane first (GpuANSDecode.h:78-92). Every lane loads (a lane
+// that reads nothing, its next word): a predicated load takes more
+// instructions. A lane's load may lie one word past the words, which is the
+// warp's own memory still.
+__device__ __forceinline__ void dec_read(uint32_t& x, uint32_t& wa, uint32_t gemask) {
+  asm volatile(
+      "{\n .reg .pred p;\n .reg .b32 v, r, w;\n"
+      " setp.lt.u32 p, %0, 32768;\n"
+      " vote.sync.ballot.b32 v, p, 0xffffffff;\n"
+      " and.b32 r, v, %2;\n popc.b32 r, r;\n mad.lo.u32 r, r, -2, %1;\n"
+      " ld.shared.u16 w, [r];\n"
+      " popc.b32 v, v;\n mad.lo.u32 %1, v, -2, %1;\n"
+      " @p prmt.b32 %0, w, %0, 0x5410;\n}\n"
+      : "+r"(x), "+r"(wa) : "r"(gemask) : "memory");
+}
+
+// A block's entry and start state, checked against the stream's header.
+struct DecBlock {
+  const uint16_t* words;
+  uint32_t nw, bs, x;
+  __device__ __forceinline__ bool load(const uint8_t* __restrict__ in, uint32_t nb, uint32_t n,
+                                       uint32_t cw, uint32_t b, int lane) {
+    const uint32_t* states = reinterpret_cast<const uint32_t*>(in + kAnsHeaderBytes + 2 * kAnsSyms);
+    x = __ldg(states + (uint64_t)b * 32 + lane);
+    const uint2 bw = __ldg(reinterpret_cast<const uint2*>(states + 32ull * nb) + b);
+    const uint32_t pre = bw.y;
+    nw = bw.x & 0xffffu;
+    bs = bw.x >> 16;
+    words = reinterpret_cast<const uint16_t*>(in + ans_overhead(nb)) + pre;
+    const uint32_t expect = (b + 1 == nb) ? n - b * kAnsBlock : kAnsBlock;
+    const uint32_t padded = (nw + 7) & ~7u;
+    return bs == expect && (uint64_t)pre + padded <= cw && padded <= kEncOutWords && !(pre & 7);
+  }
+};
+
+// One step's lookup: slot of the state, table entry, new state.
 template <int kP>
-__device__ __forceinline__ bool decode_full_smem(uint32_t x, uint32_t wa, uint32_t wa_end,
-                                                 uint32_t lut, uint8_t* __restrict__ dst,
-                                                 uint8_t* ostage, int lane) {
-  constexpr uint32_t kMask = (1u << kP) - 1u;
-  const uint32_t ltmask = lanemask_lt();
-  const uint32_t ph = phase16(dst);  // dst + 512 c has the same phase
-  uint8_t* st = ostage + ph + lane;
+__device__ __forceinline__ uint32_t dec_lookup(uint32_t& x, const uint8_t* lut_lane) {
+  constexpr uint32_t kShift = dec_copy_bits(kP) + 3, kMask = ((1u << kP) - 1u) << kShift;
+  const uint2 e = *reinterpret_cast<const uint2*>(lut_lane + ((x << kShift) & kMask));
+  asm("mad.hi.u32 %0, %0, %1, %2;" : "+r"(x) : "r"(e.x), "r"((uint32_t)((int)e.y >> 8)));
+  return e.y;
+}
+
+// Decode kBlocks (1 or 2) consecutive blocks, b on, of one stream (one warp)
+// into out + 4096 b. in: the stream (header validated by the caller: nb
+// blocks, n bytes, cw words); lut: its slot table for precision kP. A step is a chain of two shared-memory loads, a vote and
+// a population count; two blocks at a time give the warp two chains. With
+// kBlocks = 2 both blocks are full.
+// A corrupt stream can move the window's wa below the warp's words, by at most
+// 128 steps x 32 words = 8 KiB; the slot table (128 KiB) lies below
+// every warp's words in the CTA's shared memory, so such reads stay inside it,
+// and the final position check reports the block.
+// Stage: DecWarp (kBlocks of them) or DecWhole, the warp's shared memory.
+// hook(c) runs before chunk c (the block's chunks count down to 0); bad(b) in
+// lane 0 reports block b as corrupt.
+template <int kP, int kBlocks, typename Stage, typename Hook, typename Bad>
+__device__ __forceinline__ void decode_block(const uint8_t* __restrict__ in, uint32_t nb, uint32_t n,
+                                             uint32_t cw, uint8_t* __restrict__ out,
+                                             const uint8_t* lut, Stage* ws, uint32_t b, int lane,
+                                             Hook hook, Bad bad) {
+  DecBlock k[kBlocks];
+  bool fits = true;
+#pragma unroll
+  for (int u = 0; u < kBlocks; ++u) {
+    const bool f = k[u].load(in, nb, n, cw, b + u, lane);
+    if (!f && lane == 0) bad(b + u);
+    fits = fits && f;
+  }
+  if (!fits) return;
+  uint8_t* dst = out + (uint64_t)b * kAnsBlock;
+  const uint32_t gemask = lanemask_ge();
+  const uint8_t* const ll = lut + 8u * (lane & ((1 << dec_copy_bits(kP)) - 1));
+  DecWindow w[kBlocks];
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < kBlocks; ++u) {
+    if (Stage::kWhole) w[u].open_whole(k[u].words, k[u].nw, ws[u].words, lane);
+    else w[u].open(k[u].words, k[u].nw, ws[u].words, lane);
+  }
+  __syncwarp();
+  int chunks = kAnsStepsPerBlock / kDecChunkSteps;
+  if (kBlocks == 1) {
+    const uint32_t bs = k[0].bs;
+    chunks = (int)(bs / kDecChunkBytes);
+    // a last block's other steps, one by one
+    for (int j = (int)((bs + 31) >> 5) - 1; j >= chunks * kDecChunkSteps; --j) {
+      if (!Stage::kWhole) w[0].advance(lane);
+      uint32_t xs = kAnsStartState;  // a lane without a symbol reads nothing
+      const bool valid = 32u * j + lane < bs;
+      if (valid) {
+        xs = k[0].x;
+        dst[j * 32 + lane] = (uint8_t)dec_lookup<kP>(xs, ll);
+      }
+      dec_read(xs, w[0].wa, gemask);
+      if (valid) k[0].x = xs;
+    }
+  }
+  const uint32_t ph = phase16(dst);  // the phase of every chunk
 #pragma unroll 1
-  for (int c = kAnsStepsPerBlock / kDecChunkSteps - 1; c >= 0; --c) {
+  for (int c = chunks - 1; c >= 0; --c) {
+    hook(c);
 #pragma unroll
     for (int i = kDecChunkSteps - 1; i >= 0; --i) {
-      const uint32_t e = ld_shared_u32(lut + ((x & kMask) << 2));
-      st[i * 32] = (uint8_t)e;
-      x = (e >> 20) * (x >> kP) + ((e >> 8) & 0xfffu);
-      const bool rd = x < kAnsStartState;
-      const uint32_t vote = __ballot_sync(0xffffffffu, rd);
-      wa -= 2u * __popc(vote);
-      if (rd) x = (x << 16) | ld_shared_u16(wa + 2u * __popc(vote & ltmask));
-    }
-    __syncwarp();
-    dec_flush_chunk(dst + kDecChunkBytes * c, ostage, ph, lane);
-    __syncwarp();
-  }
-  return wa == wa_end && x == kAnsStartState;
-}
-
-// Any block (partial last block, or words in global memory): the same steps
-// with byte stores and a clamped word index. words: the block's first word
-// (shared or global); ptr: its word count.
-__device__ __forceinline__ bool decode_any(uint32_t x, const uint16_t* words, int ptr, uint32_t bs,
-                                           int p, const uint32_t* lut, uint8_t* __restrict__ dst,
-                                           int lane) {
-  const uint32_t mask = (1u << p) - 1u;
-  const uint32_t gemask = lanemask_ge();
-  const uint32_t rem = bs & 31;
-  int j = (int)((bs + 31) >> 5) - 1;
-  for (; j >= 0; --j) {
-    const bool valid = rem == 0 || j < (int)(bs >> 5) || (uint32_t)lane < rem;
-    if (valid) {
-      const uint32_t e = lut[x & mask];
-      dst[j * 32 + lane] = (uint8_t)e;
-      x = (e >> 20) * (x >> p) + ((e >> 8) & 0xfffu);
-    }
-    const bool rd = valid && x < kAnsStartState;
-    const uint32_t vote = __ballot_sync(0xffffffffu, rd);
-    // a read below the block's first word only happens in a corrupt stream;
-    // it is clamped here and caught by the final position check
-    if (rd) x = x * 65536u + words[max(ptr - __popc(vote & gemask), 0)];
-    ptr -= __popc(vote);
-  }
-  return ptr == 0 && x == kAnsStartState;
-}
-
-// Decode block b of one stream (one warp) into out + 4096 b. in: the stream
-// (header validated by the caller: nb blocks, n bytes, cw words, precision
-// p); lut: the slot table in shared memory (2^11 words, placed below every
-// warp's stage); ws / bar / parity: the warp's stage and its mbarrier.
-__device__ __forceinline__ void decode_block(const uint8_t* __restrict__ in, uint32_t nb,
-                                             uint32_t n, uint32_t cw, int p,
-                                             uint8_t* __restrict__ out, const uint32_t* lut,
-                                             DecWarpSmem* ws, uint64_t* bar, uint32_t& parity,
-                                             const Sink& sink, uint32_t b, int lane) {
-  const uint64_t over = ans_overhead(nb);
-  const uint32_t* states = reinterpret_cast<const uint32_t*>(in + kAnsHeaderBytes + 2 * kAnsSyms);
-  const uint2* bwords = reinterpret_cast<const uint2*>(in + kAnsHeaderBytes + 2 * kAnsSyms + 128ull * nb);
-  const uint16_t* data = reinterpret_cast<const uint16_t*>(in + over);
-  const uint32_t x = __ldg(states + (uint64_t)b * 32 + lane);
-  const uint2 bw = __ldg(bwords + b);
-  const uint32_t bs = bw.x >> 16, nw = bw.x & 0xffffu, pre = bw.y;
-  const uint32_t expect = (b + 1 == nb) ? n - b * kAnsBlock : kAnsBlock;
-  const uint32_t padded = (nw + 7) & ~7u;
-  if (bs != expect || (uint64_t)pre + padded > cw || padded > kEncOutWords || (pre & 7)) {
-    if (lane == 0) report(sink, MANS_ERR_CORRUPT, b);
-    return;
-  }
-  uint8_t* dst = out + (uint64_t)b * kAnsBlock;
-  bool ok;
-  if (padded <= kDecStageWords) {
-    // stage the block's words with one bulk copy (16-byte aligned: over % 16
-    // == 0, pre % 8 == 0); the previous block's reads of the stage are done
-    __syncwarp();
-    if (padded) {
-      if (lane == 0) bulk_load(ws->words, data + pre, 2 * padded, bar);
-      if (!mbar_wait(bar, parity) && lane == 0) report(sink, MANS_ERR_TIMEOUT, b);
-      parity ^= 1u;
-    }
-    if (bs == kAnsBlock) {
-      const uint32_t w0 = smem_addr(ws->words), l0 = smem_addr(lut);
-      switch (p) {
-        case 9: ok = decode_full_smem<9>(x, w0 + 2 * nw, w0, l0, dst, ws->out, lane); break;
-        case 10: ok = decode_full_smem<10>(x, w0 + 2 * nw, w0, l0, dst, ws->out, lane); break;
-        default: ok = decode_full_smem<11>(x, w0 + 2 * nw, w0, l0, dst, ws->out, lane); break;
+      if (!Stage::kWhole && (i & 7) == 7) {
+#pragma unroll
+        for (int u = 0; u < kBlocks; ++u) w[u].advance(lane);
       }
-    } else {
-      ok = decode_any(x, ws->words, (int)nw, bs, p, lut, dst, lane);
+#pragma unroll
+      for (int u = 0; u < kBlocks; ++u)
+        ws[u].out[ph + lane + i * 32] = (uint8_t)dec_lookup<kP>(k[u].x, ll);
+#pragma unroll
+      for (int u = 0; u < kBlocks; ++u) dec_read(k[u].x, w[u].wa, gemask);
     }
-  } else {
-    ok = decode_any(x, data + pre, (int)nw, bs, p, lut, dst, lane);
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < kBlocks; ++u)
+      dec_flush_chunk(dst + u * kAnsBlock + kDecChunkBytes * c, ws[u].out, ph, lane);
+    __syncwarp();
   }
-  if (__any_sync(0xffffffffu, !ok) && lane == 0) report(sink, MANS_ERR_CORRUPT, b);
+#pragma unroll
+  for (int u = 0; u < kBlocks; ++u) {
+    const bool ok = w[u].base == 0 && w[u].wa == w[u].wb && k[u].x == kAnsStartState;
+    if (__any_sync(0xffffffffu, !ok) && lane == 0) bad(b + u);
+  }
 }
 
 }  // namespace mans

@@ -15,7 +15,7 @@
 // per buffer; raw-byte buffers are only histogrammed) -> plan (one CTA per
 // buffer: normalise, scan of block counts across buffers, header of empty
 // buffers) -> encode. Decompress: begin -> plan (validate headers, scan of
-// decode chunks) -> decode (a CTA takes a chunk of up to 32 blocks of one
+// decode chunks) -> decode (a CTA takes a chunk of blocks of one
 // buffer and keeps that buffer's decode table in shared memory) -> unmap.
 // Every stage reads its bounds from device memory, and the look-back epoch is
 // device-resident, so a whole batch can be captured in a CUDA graph.
@@ -29,6 +29,8 @@ namespace mans {
 
 constexpr int kBWarps = 8;
 constexpr int kBThreads = kBWarps * 32;
+constexpr int kDWarps = 32;  // decode: one CTA per SM around one replicated table
+constexpr int kDThreads = kDWarps * 32;
 constexpr uint32_t kRawChunk = 4096;  // histogram unit of a raw-byte buffer
 
 __device__ __forceinline__ Sink item_sink(Ctrl* ctrl, BatchState* st) {
@@ -505,17 +507,13 @@ __global__ __launch_bounds__(kBThreads, 4) void batch_encode_kernel(const BatchI
 
 // ------------------------------------------------------------------------
 // Decompress stage 1: per buffer, validate the header and scan the decode
-// chunks (32 blocks each) across buffers.
+// chunks (chunk_blocks blocks each) across buffers.
 // ------------------------------------------------------------------------
-// Four blocks per warp per chunk: the CTA's barriers between chunks wait for
-// its slowest warp, and longer chunks even the warps out (4,096 mixed
-// buffers: decode stage 21.5 ms with one block per warp, 20.4 with four).
-constexpr uint32_t kChunkBlocks = 4 * kBWarps;
-
 __global__ __launch_bounds__(32) void batch_plan_decode_kernel(const BatchItem* __restrict__ items,
                                                                BatchState* states, uint32_t count,
                                                                Ctrl* ctrl,
-                                                               unsigned long long* item_flags) {
+                                                               unsigned long long* item_flags,
+                                                               uint32_t chunk_blocks) {
   const int lane = threadIdx.x;
   const uint32_t epoch = *((volatile uint32_t*)&ctrl->epoch);
   while (true) {
@@ -541,7 +539,7 @@ __global__ __launch_bounds__(32) void batch_plan_decode_kernel(const BatchItem* 
       if (lane == 0) report(sink, MANS_ERR_WORKSPACE_OVERFLOW, n);
       ok = false;
     }
-    const uint32_t chunks = ok ? (nb + kChunkBlocks - 1) / kChunkBlocks : 0u;
+    const uint32_t chunks = ok ? (nb + chunk_blocks - 1) / chunk_blocks : 0u;
     if (lane == 0) st_flag(&item_flags[i], make_flag(i == 0 ? kFlagIncl : kFlagAgg, epoch, chunks));
     uint32_t excl = 0;
     if (i > 0) {
@@ -573,87 +571,126 @@ __global__ __launch_bounds__(32) void batch_plan_decode_kernel(const BatchItem* 
 }
 
 // ------------------------------------------------------------------------
-// Decompress stage 2: a CTA claims a chunk of up to 32 blocks of one buffer;
-// warp w decodes blocks 32c + w + 8k, k = 0..3. The decode tables of the CTA's current
-// buffer stay in shared memory until the CTA moves to another buffer.
+// Decompress stage 2: a CTA of 32 warps claims a chunk of one buffer's blocks
+// and decodes it with the buffer's table, replicated as in the single-buffer
+// decoder (built anew when the CTA moves to another buffer). chunk_blocks: 128
+// (two pairs of blocks per warp) where the batch has blocks enough, since the
+// CTA's barriers between chunks wait for its slowest warp; down to 8 for
+// small batches, which spreads their blocks over the SMs. (256 mixed buffers,
+// 1.6 GB: 0.985 ms; CTAs of 8 warps with one copy of a 4-byte table, 1.142.)
 // ------------------------------------------------------------------------
+struct BatchChunk {
+  const uint8_t* in;  // the buffer's stream
+  uint8_t* out;       // its decoded bytes
+  uint32_t nb, n, cw, p;
+  uint32_t b0, b1;    // the chunk's blocks (b0 = b1: no more chunks)
+  uint32_t item;
+};
 struct BatchDecSmem {
-  uint32_t lut[1 << kMaxProbBits];  // below every warp's stage (see decode_full_smem)
-  DecWarpSmem warp[kBWarps];
-  uint64_t bar[kBWarps];
+  alignas(16) uint8_t lut[kDecLutBytes];  // below every warp's words (see decode_block)
+  DecWarp warp[kDWarps][2];
 };
 
-__global__ __launch_bounds__(kBThreads) void batch_decode_kernel(const BatchItem* __restrict__ items,
-                                                                 BatchState* states, uint32_t count,
-                                                                 Ctrl* ctrl) {
+// Decode the warp's blocks of a chunk. The descriptor stays in shared memory
+// and is read block by block, which keeps it out of the coder's registers.
+template <int kP, typename Bad>
+__device__ __forceinline__ void batch_decode_chunk(const volatile BatchChunk& d, const uint8_t* lut,
+                                                   DecWarp* ws, bool pairs, int warp, int lane,
+                                                   Bad bad) {
+  const uint32_t step = pairs ? 2u : 1u;
+  for (uint32_t b = d.b0 + step * warp; b < d.b1; b += step * kDWarps) {
+    if (pairs && b + 2 < d.nb && b + 2 <= d.b1) {
+      decode_block<kP, 2>(d.in, d.nb, d.n, d.cw, d.out, lut, ws, b, lane, [](int) {}, bad);
+    } else {
+#pragma unroll 1
+      for (uint32_t k = b; k < d.b1 && k < b + step; ++k)
+        decode_block<kP, 1>(d.in, d.nb, d.n, d.cw, d.out, lut, ws, k, lane, [](int) {}, bad);
+    }
+  }
+}
+
+__global__ __launch_bounds__(kDThreads, 1) void batch_decode_kernel(const BatchItem* __restrict__ items,
+                                                                    BatchState* states, uint32_t count,
+                                                                    Ctrl* ctrl,
+                                                                    uint32_t chunk_blocks) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   BatchDecSmem& sm = *reinterpret_cast<BatchDecSmem*>(smem_raw);
-  __shared__ uint32_t s_scan[kBWarps];
-  __shared__ uint32_t s_claim[2];
-  __shared__ int s_last, s_tables;
+  __shared__ uint32_t s_incl[kAnsSyms];
+  __shared__ BatchChunk s_chunk[3];
+  __shared__ uint32_t s_item, s_tables, s_cur;
+  __shared__ int s_last;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  uint64_t* bar = &sm.bar[warp];
-  if (lane == 0) mbar_init(bar);
-  uint32_t parity = 0;
-  const uint64_t total = __ldcg(&ctrl->merged_size);
-  uint32_t it = 0, pit = 0, cur_item = 0xffffffffu;
+  const bool pairs = chunk_blocks > (uint32_t)kDWarps;
   auto base = [&](uint32_t i) { return (uint64_t)states[i].unit_base; };
-  // Chunks are claimed two ahead: while chunk c is decoded, thread 0 claims
-  // the chunk after next (its atomic's latency is hidden) and every warp
-  // prefetches into L2 the words of its block of the next chunk.
-  // Every barrier in the loop below is reached by all threads: c and nxt are
-  // read from shared memory between two barriers, so they are the same in
-  // every thread, and thread 0 writes a claim only after all have read.
+  // Claim a chunk and describe it (thread 0).
+  auto claim = [&](uint32_t slot) {
+    BatchChunk& d = s_chunk[slot];
+    const uint32_t c = atomicAdd(&ctrl->tile_counter[1], 1u);
+    d.b0 = d.b1 = 0;
+    if (c >= __ldcg(&ctrl->merged_size)) return;
+    const uint32_t it = find_item(s_item, count, c, base);
+    s_item = it;
+    const BatchItem& b = items[it];
+    const BatchState& st = states[it];
+    d.in = b.in;
+    d.out = b.dtype == MANS_U8 ? b.out : b.m;
+    d.nb = st.nb;
+    d.n = st.n_hdr;
+    d.cw = st.cw;
+    d.p = st.p;
+    d.b0 = (c - st.unit_base) * chunk_blocks;
+    d.b1 = min(d.b0 + chunk_blocks, d.nb);
+    d.item = it;
+  };
+  // Chunks are described two ahead: while chunk i is decoded, thread 0 claims
+  // chunk i + 2 and every warp prefetches into L2 the words of its blocks of
+  // chunk i + 1. Every barrier in the loop is reached by all threads: what
+  // they branch on is written before a barrier and read after it.
   if (t == 0) {
-    s_claim[0] = atomicAdd(&ctrl->tile_counter[1], 1u);
-    s_claim[1] = atomicAdd(&ctrl->tile_counter[1], 1u);
+    s_item = 0;
+    s_cur = 0xffffffffu;
+    s_tables = 0;
+    claim(0);
+    claim(1);
   }
   __syncthreads();
-  uint32_t c = s_claim[0], nxt = s_claim[1];
-  __syncthreads();  // all have read both claims before thread 0 writes the next
-  while (c < total) {
-    if (t == 0) s_claim[0] = atomicAdd(&ctrl->tile_counter[1], 1u);  // read after the barrier below
-    if (nxt < total && lane == 0) {
-      pit = find_item(pit, count, nxt, base);
-      const BatchState* ps = &states[pit];
-      for (uint32_t k = 0; k < kChunkBlocks / kBWarps; ++k) {
-        const uint32_t pblk = (nxt - ps->unit_base) * kChunkBlocks + warp + k * kBWarps;
-        if (pblk < ps->nb) {
-          const uint8_t* pin = items[pit].in;
-          const uint2 bw = __ldg(reinterpret_cast<const uint2*>(
-                                     pin + kAnsHeaderBytes + 2 * kAnsSyms + 128ull * ps->nb) +
-                                 pblk);
-          const uint32_t wn = ((bw.x & 0xffffu) + 7) & ~7u;
-          if ((uint64_t)bw.y + wn <= ps->cw)
-            prefetch_l2(pin + ans_overhead(ps->nb) + 2ull * bw.y, 2 * wn);
-        }
-      }
-    }
-    it = find_item(it, count, c, base);  // uniform across the CTA
-    const BatchItem& b = items[it];
-    BatchState* st = &states[it];
-    const uint32_t p = st->p;
-    if (it != cur_item) {
-      const bool ok = build_decode_tables(b.in, (int)p, sm.lut, s_scan);
+  for (uint32_t i = 0;; i = i == 2 ? 0 : i + 1) {
+    const volatile BatchChunk& d = s_chunk[i];
+    if (d.b0 == d.b1) break;
+    if (s_cur != d.item) {
+      const bool ok = dec_build_lut(dec_pdf(d.in), (int)d.p, sm.lut, s_incl);
       if (t == 0) s_tables = ok;
       __syncthreads();
-      if (!s_tables && t == 0) report(item_sink(ctrl, st), MANS_ERR_BAD_STREAM, it);
-      cur_item = it;
-    }
-    if (s_tables) {
-      for (uint32_t k = 0; k < kChunkBlocks / kBWarps; ++k) {
-        const uint32_t blk = (c - st->unit_base) * kChunkBlocks + warp + k * kBWarps;
-        if (blk < st->nb) {
-          uint8_t* dst = b.dtype == MANS_U8 ? b.out : b.m;
-          decode_block(b.in, st->nb, st->n_hdr, st->cw, (int)p, dst, sm.lut, &sm.warp[warp], bar,
-                       parity, item_sink(ctrl, st), blk, lane);
-        }
+      if (t == 0) {
+        s_cur = d.item;
+        if (!ok) report(item_sink(ctrl, &states[d.item]), MANS_ERR_BAD_STREAM, d.item);
       }
     }
-    __syncthreads();  // the chunk is done (the table may be rebuilt); s_claim[0] is set
-    c = nxt;
-    nxt = s_claim[0];
-    __syncthreads();  // everyone has read s_claim[0] before thread 0 overwrites it
+    if (t == 0) claim(i == 0 ? 2 : i - 1);
+    {
+      const volatile BatchChunk& e = s_chunk[i == 2 ? 0 : i + 1];
+      // the warp's blocks of the next chunk: pairs at 2 (warp + 32 m), or one
+      const uint32_t k = e.b0 + (pairs ? 2u * warp + (lane & 1) + 64u * (lane >> 1)
+                                       : (uint32_t)(warp + 32 * lane));
+      if (lane < 4 && k < e.b1) {
+        const uint8_t* pst = e.in + kAnsHeaderBytes + 2 * kAnsSyms;
+        const uint32_t nb = e.nb;
+        const uint2 bw = __ldg(reinterpret_cast<const uint2*>(pst + 128ull * nb) + k);
+        const uint32_t wn = ((bw.x & 0xffffu) + 7) & ~7u;
+        if ((uint64_t)bw.y + wn <= e.cw) prefetch_l2(e.in + ans_overhead(nb) + 2ull * bw.y, 2 * wn);
+        prefetch_l2(pst + 128ull * k, 128);
+      }
+    }
+    if (s_tables) {
+      DecWarp* const ws = sm.warp[warp];
+      auto bad = [&](uint32_t k) { report(item_sink(ctrl, &states[d.item]), MANS_ERR_CORRUPT, k); };
+      switch (d.p) {
+        case 9: batch_decode_chunk<9>(d, sm.lut, ws, pairs, warp, lane, bad); break;
+        case 10: batch_decode_chunk<10>(d, sm.lut, ws, pairs, warp, lane, bad); break;
+        default: batch_decode_chunk<11>(d, sm.lut, ws, pairs, warp, lane, bad);
+      }
+    }
+    __syncthreads();  // the chunk is done (the table may be rebuilt)
   }
   __syncthreads();
   if (t == 0) {
@@ -785,7 +822,7 @@ void init_batch_cfg(BatchCfg& c, const LaunchCfg& base) {
   c.occ[kStagePlanEnc] = occ((const void*)batch_plan_encode_kernel, 256, 0);
   c.occ[kStageEncode] = occ((const void*)batch_encode_kernel, kBThreads, sizeof(BatchEncSmem));
   c.occ[kStagePlanDec] = occ((const void*)batch_plan_decode_kernel, 32, 0);
-  c.occ[kStageDecode] = occ((const void*)batch_decode_kernel, kBThreads, sizeof(BatchDecSmem));
+  c.occ[kStageDecode] = occ((const void*)batch_decode_kernel, kDThreads, sizeof(BatchDecSmem));
   c.occ[kStageUnmap] = min(occ((const void*)batch_unmap_kernel<MANS_U16>, kBThreads, 0),
                            occ((const void*)batch_unmap_kernel<MANS_U32>, kBThreads,
                                sizeof(BatchUnmapSmem)));
@@ -854,15 +891,20 @@ cudaError_t launch_batch_compress(const BatchDev& d, uint32_t count, const uint6
 }
 
 cudaError_t launch_batch_decompress(const BatchDev& d, uint32_t count, const uint64_t groups[3],
-                                    uint64_t max_chunks, const BatchCfg& c, cudaStream_t s,
-                                    cudaEvent_t* marks) {
+                                    uint64_t likely_blocks, uint64_t max_blocks, const BatchCfg& c,
+                                    cudaStream_t s, cudaEvent_t* marks) {
+  uint32_t chunk = 8;
+  while (chunk < (uint32_t)kDWarps && likely_blocks > (uint64_t)c.sms * chunk) chunk *= 2;
+  if (likely_blocks >= (uint64_t)c.sms * 2 * 64) chunk = 64;
+  if (likely_blocks >= (uint64_t)c.sms * 4 * 128) chunk = 128;
+  const uint64_t max_chunks = div_up_u64(max_blocks, chunk) + count;
   if (marks) cudaEventRecord(marks[0], s);
   batch_begin_kernel<<<(count + 255) / 256 + 1, 256, 0, s>>>(d.states, count, d.ctrl);
   batch_plan_decode_kernel<<<grid_of(c, kStagePlanDec, count), 32, 0, s>>>(
-      d.items, d.states, count, d.ctrl, d.item_flags);
+      d.items, d.states, count, d.ctrl, d.item_flags, chunk);
   if (marks) cudaEventRecord(marks[1], s);
-  batch_decode_kernel<<<grid_of(c, kStageDecode, max_chunks), kBThreads, sizeof(BatchDecSmem),
-                        s>>>(d.items, d.states, count, d.ctrl);
+  batch_decode_kernel<<<grid_of(c, kStageDecode, max_chunks), kDThreads, sizeof(BatchDecSmem),
+                        s>>>(d.items, d.states, count, d.ctrl, chunk);
   if (marks) cudaEventRecord(marks[2], s);
   if (groups[1])
     batch_unmap_kernel<MANS_U16><<<grid_of(c, kStageUnmap, div_up_u64(groups[1], kBWarps),

@@ -60,8 +60,9 @@ namespace {
 
 // Lay out one call's buffers: fills `h` (count descriptors) and the totals.
 mans_status layout(mans_batch* b, const mans_batch_item* items, uint32_t count, bool compress,
-                   BatchItem* h, uint64_t groups[3], uint64_t* max_units, uint64_t* max_chunks) {
-  uint64_t off = 0, flags = 0, units = 0, chunks = 0, total = 0;
+                   BatchItem* h, uint64_t groups[3], uint64_t* max_units,
+                   uint64_t* likely_units) {
+  uint64_t off = 0, flags = 0, units = 0, likely = 0, total = 0;
   groups[0] = groups[1] = groups[2] = 0;
   for (uint32_t i = 0; i < count; ++i) {
     const mans_batch_item& it = items[i];
@@ -96,9 +97,8 @@ mans_status layout(mans_batch* b, const mans_batch_item* items, uint32_t count, 
       blocks = div_up_u64(bytes, kAnsBlock);
     } else {
       g = div_up_u64(it.n_elems, kAdmGroup);
-      const uint64_t hdr = it.dtype == MANS_U16 ? 6 * g : 40 * g;
       const uint64_t cap = std::min(mapped_cap(bytes, b->ratio_pct), kMaxMerged);
-      d.m = b->pool + off + merged_pad(hdr);
+      d.m = b->pool + off + (it.dtype == MANS_U16 ? merged_pad(6 * g) : 0);
       d.m_cap = cap;
       off += align_up(cap + kItemSlack, 256);
       blocks = div_up_u64(cap, kAnsBlock);
@@ -109,14 +109,15 @@ mans_status layout(mans_batch* b, const mans_batch_item* items, uint32_t count, 
     groups[kind] += claims;
     flags += claims;
     units += blocks;
-    chunks += div_up_u64(blocks, 8);
+    // an element maps to one byte, and a little more
+    likely += it.dtype == MANS_U8 ? blocks : div_up_u64(it.n_elems + it.n_elems / 4, kAnsBlock);
   }
   if (total > b->max_total_bytes || off > b->pool_bytes || flags > b->group_flags_n ||
       units > b->block_flags_n || groups[0] >= (1ull << 32) || groups[1] >= (1ull << 32) ||
       groups[2] >= (1ull << 32))
     return MANS_ERR_TOO_LARGE;
   *max_units = units;
-  *max_chunks = chunks;
+  *likely_units = likely;
   return MANS_OK;
 }
 
@@ -156,8 +157,8 @@ mans_status run(mans_batch* b, const mans_batch_item* items, uint32_t count, boo
   if (count > b->max_items) return MANS_ERR_TOO_LARGE;
   if (count == 0) return MANS_OK;
   std::vector<BatchItem> h(count);
-  uint64_t groups[3], units = 0, chunks = 0;
-  mans_status st = layout(b, items, count, compress, h.data(), groups, &units, &chunks);
+  uint64_t groups[3], units = 0, likely = 0;
+  mans_status st = layout(b, items, count, compress, h.data(), groups, &units, &likely);
   if (st != MANS_OK) return st;
   st = upload(b, h.data(), count, s);
   if (st != MANS_OK) return st;
@@ -170,8 +171,8 @@ mans_status run(mans_batch* b, const mans_batch_item* items, uint32_t count, boo
     if (cap == cudaStreamCaptureStatusNone) marks = b->marks[dir][b->recorded[dir]++];
   }
   cudaError_t e = compress ? launch_batch_compress(b->dev, count, groups, units, b->cfg, s, marks)
-                           : launch_batch_decompress(b->dev, count, groups, chunks, b->cfg, s,
-                                                     marks);
+                           : launch_batch_decompress(b->dev, count, groups, likely, units, b->cfg,
+                                                     s, marks);
   return e == cudaSuccess ? MANS_OK : MANS_ERR_CUDA;
 }
 

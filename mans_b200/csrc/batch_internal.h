@@ -70,7 +70,8 @@ enum BatchStage {
 // Schedule of the batched kernels. The bytes produced do not depend on it.
 //   ctas_per_sm: resident CTAs per SM of each stage (<= occ); for the map
 //     stage counted in CTAs of 8 warps, whatever its warps per CTA.
-//   warps: warps per CTA (the map stage takes 4 or 8; the others 8).
+//   warps: warps per CTA (the map stage takes 4 or 8; the others have a fixed
+//     number, shown as 8).
 //   prefetch: L2 prefetch distance of the map and encode stages, in grids of
 //     units ahead (0: none; at most kMaxPrefetch).
 struct BatchCfg {
@@ -97,8 +98,8 @@ cudaError_t launch_batch_compress(const BatchDev& d, uint32_t count, const uint6
                                   uint64_t max_blocks, const BatchCfg& c, cudaStream_t s,
                                   cudaEvent_t* marks = nullptr);
 cudaError_t launch_batch_decompress(const BatchDev& d, uint32_t count, const uint64_t groups[3],
-                                    uint64_t max_chunks, const BatchCfg& c, cudaStream_t s,
-                                    cudaEvent_t* marks = nullptr);
+                                    uint64_t likely_blocks, uint64_t max_blocks, const BatchCfg& c,
+                                    cudaStream_t s, cudaEvent_t* marks = nullptr);
 cudaError_t launch_batch_gather_status(const BatchDev& d, uint32_t count, uint32_t* status,
                                        unsigned long long* detail, cudaStream_t s);
 inline int dtype_kind(uint32_t dtype) { return dtype == 1 ? 0 : dtype == 2 ? 1 : 2; }

@@ -204,9 +204,9 @@ mans_status compress_impl(mans_workspace* ws, mans_dtype dtype, mans_layout layo
     e = launch_adm_u16_map((const uint16_t*)d_in, n_elems, m, ws->merged_cap, ws->ctrl,
                            ws->adm_flags, precision, ws->cfg, s, (int)layout);
   } else {
-    const uint64_t hdr = adm_u32_header_bytes(n_elems);
-    if (hdr + n_elems > ws->merged_cap) return MANS_ERR_TOO_LARGE;
-    m = ws->merged + merged_pad(hdr);
+    // 16-byte aligned; the records (40 bytes a group on) are then 8-byte aligned
+    if (adm_u32_header_bytes(n_elems) + n_elems > ws->merged_cap) return MANS_ERR_TOO_LARGE;
+    m = ws->merged;
     e = launch_adm_u32_map((const uint32_t*)d_in, n_elems, m, ws->merged_cap, ws->ctrl,
                            ws->adm_flags, precision, ws->cfg, s);
   }
@@ -244,14 +244,14 @@ mans_status decompress_impl(mans_workspace* ws, mans_dtype dtype, mans_layout la
   mark(ws, 3, s);
   if (dtype == MANS_U8) {
     e = launch_ans_decode((const uint8_t*)d_in, in_size, (uint8_t*)d_out, out_bytes, ws->ctrl, -1,
-                          0, div_up_u64(out_bytes, kAnsBlock), ws->cfg, s);
+                          0, div_up_u64(out_bytes, kAnsBlock), div_up_u64(out_bytes, kAnsBlock),
+                          ws->cfg, s);
     mark(ws, 4, s);
     mark(ws, 5, s);
     return e == cudaSuccess ? MANS_OK : MANS_ERR_CUDA;
   }
-  const uint64_t hdr = dtype == MANS_U16 ? adm_u16_header_bytes(n_elems, (int)layout)
-                                         : adm_u32_header_bytes(n_elems);
-  uint8_t* m = ws->merged + merged_pad(hdr);
+  uint8_t* m = ws->merged;
+  if (dtype == MANS_U16) m += merged_pad(adm_u16_header_bytes(n_elems, (int)layout));
   if (unmap_only) {
     if (in_size > ws->merged_cap) return MANS_ERR_TOO_LARGE;
     import_merged_kernel<<<copy_grid(ws->cfg, in_size), 256, 0, s>>>((const uint8_t*)d_in, m,
@@ -259,6 +259,7 @@ mans_status decompress_impl(mans_workspace* ws, mans_dtype dtype, mans_layout la
     e = cudaGetLastError();
   } else {
     e = launch_ans_decode((const uint8_t*)d_in, in_size, m, ws->merged_cap, ws->ctrl, -1, 1,
+                          div_up_u64(n_elems + n_elems / 4, kAnsBlock),
                           div_up_u64(ws->merged_cap, kAnsBlock), ws->cfg, s);
   }
   mark(ws, 4, s);
@@ -567,9 +568,10 @@ mans_status mans_ans_decode(int precision, const uint8_t* d_in, uint8_t* d_out,
   const WsRef ws = default_ws(s, 0, &st);
   if (!ws) return st;
   // Sizes come from the stream header on the device (as in the reference):
-  // the grid is one resident wave and the caller sized d_out from the header.
-  const uint64_t wave = (uint64_t)ws->cfg.sms * ws->cfg.dec_ctas * 4;
-  cudaError_t e = launch_ans_decode(d_in, ~0ull, d_out, ~0ull, ws->ctrl, precision, 0, wave,
+  // the grid is one resident wave of the kernel for many blocks, and the
+  // caller sized d_out from the header.
+  const uint64_t wave = (uint64_t)ws->cfg.sms * 64;
+  cudaError_t e = launch_ans_decode(d_in, ~0ull, d_out, ~0ull, ws->ctrl, precision, 0, wave, wave,
                                     ws->cfg, s);
   return e == cudaSuccess ? MANS_OK : MANS_ERR_CUDA;
 }

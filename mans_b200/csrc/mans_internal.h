@@ -23,7 +23,6 @@ struct NvtxRange {
 struct LaunchCfg {
   int sms = 148;        // multiprocessors of the device
   int enc_ctas = 0;     // resident CTAs per SM of the encode kernel (shared-memory staging)
-  int dec_ctas = 0;     // resident CTAs per SM of the decode kernel
   int map_ctas = 0;     // resident CTAs per SM of the ADM map kernels
   int map32_ctas = 0;   // resident CTAs per SM of the uint32 ADM map kernel
   int unmap32_ctas = 0; // resident CTAs per SM of the uint32 ADM unmap kernel
@@ -50,9 +49,10 @@ cudaError_t launch_ans_encode(const uint8_t* in, uint8_t* out, uint64_t out_cap,
 uint64_t ans_encode_slot_bytes(const LaunchCfg& cfg);
 // Decode the stream at `in` into `out` (at most out_cap bytes). expect_p < 0
 // accepts any valid precision. record != 0 stores the decoded size in ctrl.
+// likely_blocks and max_blocks: as in launch_ans_encode.
 cudaError_t launch_ans_decode(const uint8_t* in, uint64_t in_size, uint8_t* out, uint64_t out_cap,
-                              Ctrl* ctrl, int expect_p, int record, uint64_t max_blocks,
-                              const LaunchCfg& cfg, cudaStream_t s);
+                              Ctrl* ctrl, int expect_p, int record, uint64_t likely_blocks,
+                              uint64_t max_blocks, const LaunchCfg& cfg, cudaStream_t s);
 
 // ---- ADM uint16 (adm_u16.cu) ----
 // Map n values into the merged buffer M (16-byte aligned codes section),
@@ -75,8 +75,8 @@ cudaError_t launch_adm_u32_map(const uint32_t* in, uint64_t n, uint8_t* m, uint6
 cudaError_t launch_adm_u32_unmap(const uint8_t* m, uint64_t n, uint32_t* out, Ctrl* ctrl,
                                  const LaunchCfg& cfg, cudaStream_t s);
 
-// Byte offset of the merged buffer inside its 16-byte aligned region so that
-// the per-element section (codes / records) is 16-byte aligned.
+// Byte offset of a uint16 merged buffer inside its 16-byte aligned region so
+// that the codes are 16-byte aligned.
 inline uint64_t merged_pad(uint64_t header_bytes) { return (16 - (header_bytes & 15)) & 15; }
 inline uint64_t adm_u16_header_bytes(uint64_t n, int layout = 0) {
   const uint64_t g = (n + 511) / 512;

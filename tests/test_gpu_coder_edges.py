@@ -1,6 +1,7 @@
 """The byte coder's kernels at the sizes where their work split changes: the
-encoder's warps per CTA (4 to 32 a multiprocessor) and its word pieces of 256
-words, against the oracle, byte for byte."""
+warps per CTA (up to 32 a multiprocessor), the decoder's pairs of blocks and
+the word pieces of 256 words, and the batch decoder's chunk sizes, against the
+oracle, byte for byte."""
 import numpy as np
 import pytest
 
@@ -57,3 +58,63 @@ def test_encoder_word_pieces(ws, oracle, p):
     s = mb.compress(to_dev(x), p, ws=ws)
     np.testing.assert_array_equal(to_host(s), ref)
     np.testing.assert_array_equal(to_host(mb.decompress(s, n, torch.uint8, ws=ws)), x)
+
+
+@pytest.mark.parametrize("p", [9, 10, 11])
+@pytest.mark.parametrize("tail", [-4096 * 3 - 511, -1, 0, 1, 512, 4096])
+def test_decoder_pairs(ws, oracle, tail, p):
+    """Around two waves of pairs, through both decode calls; the last blocks
+    (one of an odd number, a partial one) are decoded singly."""
+    import torch
+    n = 2 * 64 * SMS * 4096 // 3 + tail
+    x = W.random_bytes(n, 7 + p, ("sparse", "two", "skewed")[p - 9])
+    ref = oracle.ans_encode(x, p)
+    s = to_dev(ref)
+    np.testing.assert_array_equal(to_host(mb.decompress(s, n, torch.uint8, ws=ws)), x)
+    out = torch.zeros(n, dtype=torch.uint8, device="cuda")
+    mb.ansDecode(p, s, out)
+    assert mb.ans_last_status()[0] == 0
+    np.testing.assert_array_equal(to_host(out), x)
+
+
+@pytest.mark.parametrize("n", [1 << 20, 1_000_003])
+def test_single_symbol_keeps_its_state(ws, oracle, n):
+    """A pdf of 2^p (one symbol) is the slot table's special entry."""
+    import torch
+    x = np.full(n, 200, np.uint8)
+    s = mb.compress(to_dev(x), 11, ws=ws)
+    np.testing.assert_array_equal(to_host(s), oracle.ans_encode(x, 11))
+    np.testing.assert_array_equal(to_host(mb.decompress(s, n, torch.uint8, ws=ws)), x)
+
+
+@pytest.mark.parametrize("big", [0, 900_000, 6_000_000, 24_000_000, 400_000_000])
+def test_batch_decoder_chunks(oracle, big):
+    """Chunks of 8 to 128 blocks: a few small buffers of every type and
+    precision beside one of `big` bytes that sets the chunk size."""
+    import torch
+
+    from mans_b200.batch import Batch
+    xs, ps = [], []
+    for i, n in enumerate([1, 4095, 4096 * 8 + 1, 4096 * 33, 4096 * 66 - 5, 70_001, 600_000]):
+        xs += [W.random_bytes(n, i, "skewed"), W.gradient_u16(n, i), W.quant_u32(n // 2 + 1, i)]
+        ps += [9 + i % 3] * 3
+    refs = [to_dev(oracle.ans_encode(x, p) if x.dtype == np.uint8 else oracle.compress(x, p))
+            for x, p in zip(xs, ps)]
+    tdt = {np.uint8: torch.uint8, np.uint16: torch.uint16, np.uint32: torch.uint32}
+    dt = [tdt[x.dtype.type] for x in xs]
+    big_in = None
+    if big:  # made on the device, compressed by the library itself
+        g = torch.Generator(device="cuda")
+        g.manual_seed(big)
+        big_in = torch.randint(0, 50, (big,), dtype=torch.uint8, device="cuda", generator=g)
+        refs.append(mb.compress(big_in, 10))
+        dt.append(torch.uint8)
+    sizes = [x.size for x in xs] + ([big] if big else [])
+    b = Batch(32, sum(x.nbytes for x in xs) + big)
+    try:
+        outs = b.decompress(refs, list(zip(sizes, dt)))
+        for x, y in zip(xs, outs):
+            np.testing.assert_array_equal(to_host(y, x.dtype), x)
+        assert big_in is None or torch.equal(outs[-1], big_in)
+    finally:
+        b.close()
