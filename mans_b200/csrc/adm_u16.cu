@@ -23,6 +23,7 @@ template <int kLayout>
 __global__ __launch_bounds__(kMapThreads, 4) void adm_u16_map_kernel(
     const uint16_t* __restrict__ in, uint64_t n, uint8_t* __restrict__ M, uint64_t m_cap,
     Ctrl* ctrl, unsigned long long* flags, int prob_bits) {
+  kernel_begin();
   __shared__ uint32_t s_h[kMapWarps][kAnsSyms];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   for (int i = t; i < kMapWarps * kAnsSyms; i += kMapThreads) (&s_h[0][0])[i] = 0;
@@ -100,6 +101,7 @@ template <int kLayout>
 __global__ __launch_bounds__(kUnmapThreads, 4) void adm_u16_unmap_kernel(
     const uint8_t* __restrict__ M, uint64_t n, uint16_t* __restrict__ out, Ctrl* ctrl,
     const uint32_t* __restrict__ v12_excl) {
+  kernel_begin();
   const Sink sink = sink_of(ctrl);
   if (sink_failed(sink)) return;
   const int lane = threadIdx.x & 31;
@@ -126,6 +128,7 @@ constexpr int kScanThreads = 256, kScanPer = 8, kScanTile = kScanThreads * kScan
 __global__ __launch_bounds__(kScanThreads) void adm_u16_v12_scan_kernel(
     const uint8_t* __restrict__ M, uint64_t n, uint32_t* __restrict__ excl, Ctrl* ctrl,
     unsigned long long* flags) {
+  kernel_begin();
   __shared__ uint32_t s_tile, s_warp[kScanThreads / 32], s_prefix;
   __shared__ int s_last;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -205,13 +208,10 @@ cudaError_t launch_adm_u16_map(const uint16_t* in, uint64_t n, uint8_t* m, uint6
   const uint64_t ctas = div_up_u64(div_up_u64(div_up_u64(n, kAdmGroup), kMapUnit), kMapWarps);
   const uint64_t cap = (uint64_t)cfg.sms * cfg.map_ctas;
   const unsigned grid = (unsigned)(ctas < 1 ? 1 : (ctas < cap ? ctas : cap));
-  if (layout == kLayoutV12)
-    adm_u16_map_kernel<kLayoutV12><<<grid, kMapThreads, 0, s>>>(in, n, m, m_cap, ctrl, flags, prob_bits);
-  else if (layout == kLayoutCpuV2)
-    adm_u16_map_kernel<kLayoutCpuV2><<<grid, kMapThreads, 0, s>>>(in, n, m, m_cap, ctrl, flags, prob_bits);
-  else
-    adm_u16_map_kernel<kLayoutV15><<<grid, kMapThreads, 0, s>>>(in, n, m, m_cap, ctrl, flags, prob_bits);
-  return cudaGetLastError();
+  auto* k = layout == kLayoutV12     ? adm_u16_map_kernel<kLayoutV12>
+            : layout == kLayoutCpuV2 ? adm_u16_map_kernel<kLayoutCpuV2>
+                                     : adm_u16_map_kernel<kLayoutV15>;
+  return launch(k, grid, kMapThreads, 0, s, in, n, m, m_cap, ctrl, flags, prob_bits);
 }
 
 cudaError_t launch_adm_u16_unmap(const uint8_t* m, uint64_t n, uint16_t* out, Ctrl* ctrl,
@@ -224,14 +224,14 @@ cudaError_t launch_adm_u16_unmap(const uint8_t* m, uint64_t n, uint16_t* out, Ct
   if (layout == kLayoutV12) {
     const uint64_t tiles = div_up_u64(groups, kScanTile);
     const unsigned sgrid = (unsigned)(tiles < 1 ? 1 : (tiles < (uint64_t)cfg.sms * 4 ? tiles : cfg.sms * 4));
-    adm_u16_v12_scan_kernel<<<sgrid, kScanThreads, 0, s>>>(m, n, v12_excl, ctrl, scan_flags);
-    adm_u16_unmap_kernel<kLayoutV12><<<grid, kUnmapThreads, 0, s>>>(m, n, out, ctrl, v12_excl);
-  } else if (layout == kLayoutCpuV2) {
-    adm_u16_unmap_kernel<kLayoutCpuV2><<<grid, kUnmapThreads, 0, s>>>(m, n, out, ctrl, nullptr);
-  } else {
-    adm_u16_unmap_kernel<kLayoutV15><<<grid, kUnmapThreads, 0, s>>>(m, n, out, ctrl, nullptr);
+    const cudaError_t e = launch(adm_u16_v12_scan_kernel, sgrid, kScanThreads, 0, s, m, n, v12_excl,
+                                 ctrl, scan_flags);
+    if (e != cudaSuccess) return e;
   }
-  return cudaGetLastError();
+  auto* k = layout == kLayoutV12     ? adm_u16_unmap_kernel<kLayoutV12>
+            : layout == kLayoutCpuV2 ? adm_u16_unmap_kernel<kLayoutCpuV2>
+                                     : adm_u16_unmap_kernel<kLayoutV15>;
+  return launch(k, grid, kUnmapThreads, 0, s, m, n, out, ctrl, v12_excl);
 }
 
 }  // namespace mans

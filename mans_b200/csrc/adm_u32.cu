@@ -15,6 +15,7 @@ namespace mans {
 __global__ __launch_bounds__(kMap32Threads) void adm_u32_map_kernel(
     const uint32_t* __restrict__ in, uint64_t n, uint8_t* __restrict__ M, uint64_t m_cap,
     Ctrl* ctrl, unsigned long long* flags, int prob_bits) {
+  kernel_begin();
   extern __shared__ __align__(16) uint8_t smem_raw[];
   Map32Smem& sm = *reinterpret_cast<Map32Smem*>(smem_raw);
   __shared__ uint32_t s_h[kMap32Warps][kAnsSyms];
@@ -41,6 +42,7 @@ __global__ __launch_bounds__(kMap32Threads) void adm_u32_map_kernel(
 
 __global__ __launch_bounds__(kUnmap32Threads) void adm_u32_unmap_kernel(
     const uint8_t* __restrict__ M, uint64_t n, uint32_t* __restrict__ out, Ctrl* ctrl) {
+  kernel_begin();
   extern __shared__ __align__(16) uint8_t smem_raw[];
   Unmap32Smem& sm = *reinterpret_cast<Unmap32Smem*>(smem_raw);
   const Sink sink = sink_of(ctrl);
@@ -90,18 +92,17 @@ cudaError_t launch_adm_u32_map(const uint32_t* in, uint64_t n, uint8_t* m, uint6
                                const LaunchCfg& cfg, cudaStream_t s) {
   const int occ = cfg.map32_ctas > 0 ? cfg.map32_ctas : 1;
   const uint64_t ctas = div_up_u64(div_up_u64(n, kAdmGroup), kMap32Warps);
-  adm_u32_map_kernel<<<grid_for(ctas, (uint64_t)cfg.sms * occ), kMap32Threads, sizeof(Map32Smem),
-                       s>>>(in, n, m, m_cap, ctrl, flags, prob_bits);
-  return cudaGetLastError();
+  return launch(adm_u32_map_kernel, grid_for(ctas, (uint64_t)cfg.sms * occ), kMap32Threads,
+                sizeof(Map32Smem), s, in, n, m, m_cap, ctrl, flags, prob_bits);
 }
 
 cudaError_t launch_adm_u32_unmap(const uint8_t* m, uint64_t n, uint32_t* out, Ctrl* ctrl,
                                  const LaunchCfg& cfg, cudaStream_t s) {
   const int occ = cfg.unmap32_ctas > 0 ? cfg.unmap32_ctas : 1;
   const uint64_t groups = div_up_u64(n, kAdmGroup);
-  adm_u32_unmap_kernel<<<grid_for(div_up_u64(groups, kUnmap32Warps), (uint64_t)cfg.sms * occ),
-                         kUnmap32Threads, sizeof(Unmap32Smem), s>>>(m, n, out, ctrl);
-  return cudaGetLastError();
+  return launch(adm_u32_unmap_kernel,
+                grid_for(div_up_u64(groups, kUnmap32Warps), (uint64_t)cfg.sms * occ),
+                kUnmap32Threads, sizeof(Unmap32Smem), s, m, n, out, ctrl);
 }
 
 }  // namespace mans

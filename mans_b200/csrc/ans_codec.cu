@@ -34,6 +34,7 @@ __device__ __forceinline__ void hist_word(uint32_t* h, uint32_t w) {
 __global__ __launch_bounds__(kHistThreads) void hist_bytes_kernel(const uint8_t* __restrict__ in,
                                                                   uint64_t n, Ctrl* ctrl,
                                                                   int prob_bits) {
+  kernel_begin();
   __shared__ uint32_t s_h[kHistThreads / 32][kAnsSyms];
   const int t = threadIdx.x, warp = t >> 5;
   for (int i = t; i < (kHistThreads / 32) * kAnsSyms; i += kHistThreads) (&s_h[0][0])[i] = 0;
@@ -108,6 +109,7 @@ __global__ __launch_bounds__(kEncMaxThreads, 1) void ans_encode_slots_kernel(
     const uint8_t* __restrict__ in, uint8_t* __restrict__ out, uint64_t out_cap,
     unsigned long long* out_size64, uint32_t* out_size32, Ctrl* ctrl, unsigned long long* flags,
     uint8_t* __restrict__ slots) {
+  kernel_begin();
   extern __shared__ __align__(16) uint8_t smem_raw[];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   EncWarp& sw = reinterpret_cast<EncWarp*>(smem_raw + kEncTableBytes)[warp];
@@ -165,6 +167,7 @@ __global__ __launch_bounds__(kEncThreads) void ans_encode_shared_kernel(
     const uint8_t* __restrict__ in, uint8_t* __restrict__ out, uint64_t out_cap,
     unsigned long long* out_size64, uint32_t* out_size32, Ctrl* ctrl,
     unsigned long long* flags, int p) {
+  kernel_begin();
   extern __shared__ __align__(16) uint8_t smem_raw[];
   EncSmem& ss = *reinterpret_cast<EncSmem*>(smem_raw);
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -277,6 +280,7 @@ template <int kBlocks>
 __global__ __launch_bounds__(kDecMaxWarps * 32, 1) void ans_decode_kernel(
     const uint8_t* __restrict__ in, uint64_t in_size, uint8_t* __restrict__ out, uint64_t out_cap,
     Ctrl* ctrl, int expect_p, int record, uint32_t stage_bytes) {
+  kernel_begin();
   extern __shared__ __align__(16) uint8_t smem_raw[];
   __shared__ uint32_t s_incl[kAnsSyms];
   __shared__ int s_ok;
@@ -356,8 +360,7 @@ cudaError_t launch_hist_bytes(const uint8_t* in, uint64_t n, Ctrl* ctrl, int pro
   uint64_t want = div_up_u64(n >> 4, kHistThreads);
   uint64_t cap = (uint64_t)cfg.sms * cfg.hist_ctas;
   unsigned grid = (unsigned)(want < 1 ? 1 : (want < cap ? want : cap));
-  hist_bytes_kernel<<<grid, kHistThreads, 0, s>>>(in, n, ctrl, prob_bits);
-  return cudaGetLastError();
+  return launch(hist_bytes_kernel, grid, kHistThreads, 0, s, in, n, ctrl, prob_bits);
 }
 
 uint64_t ans_encode_slot_bytes(const LaunchCfg& cfg) {
@@ -379,16 +382,15 @@ cudaError_t launch_ans_encode(const uint8_t* in, uint8_t* out, uint64_t out_cap,
     auto* k = prob_bits == 9    ? ans_encode_slots_kernel<9>
               : prob_bits == 10 ? ans_encode_slots_kernel<10>
                                 : ans_encode_slots_kernel<11>;
-    k<<<grid, (unsigned)warps * 32, enc_smem_bytes((int)warps), s>>>(
-        in, out, out_cap, out_size64, out_size32, ctrl, flags, slots);
+    return launch(k, grid, (unsigned)warps * 32, enc_smem_bytes((int)warps), s, in, out, out_cap,
+                  out_size64, out_size32, ctrl, flags, slots);
   } else {
     const uint64_t want = div_up_u64(max_blocks, kEncWarps);
     const uint64_t cap = (uint64_t)cfg.sms * cfg.enc_ctas;
     const unsigned grid = (unsigned)(want < 1 ? 1 : (want < cap ? want : cap));
-    ans_encode_shared_kernel<<<grid, kEncThreads, sizeof(EncSmem), s>>>(
-        in, out, out_cap, out_size64, out_size32, ctrl, flags, prob_bits);
+    return launch(ans_encode_shared_kernel, grid, kEncThreads, sizeof(EncSmem), s, in, out, out_cap,
+                  out_size64, out_size32, ctrl, flags, prob_bits);
   }
-  return cudaGetLastError();
 }
 
 cudaError_t launch_ans_decode(const uint8_t* in, uint64_t in_size, uint8_t* out, uint64_t out_cap,
@@ -406,9 +408,8 @@ cudaError_t launch_ans_decode(const uint8_t* in, uint64_t in_size, uint8_t* out,
       (unsigned)(want < 1 ? 1 : (want < (uint64_t)cfg.sms ? want : (uint64_t)cfg.sms));
   auto* k = blocks == 2 ? ans_decode_kernel<2> : ans_decode_kernel<1>;
   const size_t stage = dec_stage_bytes(warps, blocks);
-  k<<<grid, (unsigned)warps * 32, kDecLutBytes + stage, s>>>(in, in_size, out, out_cap, ctrl, expect_p,
-                                                             record, (uint32_t)stage);
-  return cudaGetLastError();
+  return launch(k, grid, (unsigned)warps * 32, kDecLutBytes + stage, s, in, in_size, out, out_cap,
+                ctrl, expect_p, record, (uint32_t)stage);
 }
 
 }  // namespace mans

@@ -37,6 +37,7 @@ inline uint64_t elem_bytes(uint32_t d) { return d == 1 ? 1 : d == 2 ? 2 : d == 4
 __global__ void frame_header_kernel(uint8_t* frame, uint64_t cap, uint32_t dtype, uint32_t layout,
                                     uint32_t precision, uint64_t n,
                                     unsigned long long* size_io) {
+  kernel_begin();
   const unsigned long long sz = *size_io;
   const bool ok = sz <= cap;
   const uint32_t mapped = ok && sz >= 32 ? reinterpret_cast<const uint32_t*>(frame + kFrameBytes)[2] : 0u;
@@ -114,10 +115,11 @@ mans_status mans_frame_compress(mans_workspace* ws, mans_dtype dtype, mans_layou
   mans_status st = mans_compress_ex(ws, dtype, layout, d_in, n_elems, body,
                                     out_capacity - kFrameBytes, d_out_size, precision, stream);
   if (st != MANS_OK) return st;
-  frame_header_kernel<<<1, 1, 0, s>>>(static_cast<uint8_t*>(d_out), out_capacity - kFrameBytes,
-                                      (uint32_t)dtype, (uint32_t)layout, (uint32_t)precision,
-                                      n_elems, reinterpret_cast<unsigned long long*>(d_out_size));
-  return cudaGetLastError() == cudaSuccess ? MANS_OK : MANS_ERR_CUDA;
+  const cudaError_t e =
+      launch(frame_header_kernel, 1, 1, 0, s, static_cast<uint8_t*>(d_out),
+             out_capacity - kFrameBytes, (uint32_t)dtype, (uint32_t)layout, (uint32_t)precision,
+             n_elems, reinterpret_cast<unsigned long long*>(d_out_size));
+  return e == cudaSuccess ? MANS_OK : MANS_ERR_CUDA;
 }
 
 mans_status mans_frame_decompress(mans_workspace* ws, const mans_frame_info* info,

@@ -129,6 +129,7 @@ namespace {
 // match this call's.
 __global__ void export_merged_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
                                      uint64_t cap, Ctrl* ctrl, unsigned long long* out_size) {
+  kernel_begin();
   if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->epoch = (ctrl->epoch + 1) & 0x3fffffffu;
   if (*((volatile uint32_t*)&ctrl->status) != 0) return;
   const uint64_t n = __ldcg(&ctrl->merged_size);
@@ -145,6 +146,7 @@ __global__ void export_merged_kernel(const uint8_t* __restrict__ src, uint8_t* _
 // Copy caller-supplied mapped bytes into the workspace and record their size.
 __global__ void import_merged_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
                                      uint64_t n, Ctrl* ctrl) {
+  kernel_begin();
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x)
     dst[i] = src[i];
@@ -213,9 +215,8 @@ mans_status compress_impl(mans_workspace* ws, mans_dtype dtype, mans_layout layo
   mark(ws, 1, s);
   if (e == cudaSuccess) {
     if (map_only) {
-      export_merged_kernel<<<copy_grid(ws->cfg, ws->merged_cap), 256, 0, s>>>(
-          m, (uint8_t*)d_out, out_capacity, ws->ctrl, osz);
-      e = cudaGetLastError();
+      e = launch(export_merged_kernel, copy_grid(ws->cfg, ws->merged_cap), 256, 0, s, m,
+                 (uint8_t*)d_out, out_capacity, ws->ctrl, osz);
     } else {
       // an element maps to one byte, and a little more
       e = launch_ans_encode(m, (uint8_t*)d_out, out_capacity, osz, nullptr, ws->ctrl,
@@ -254,9 +255,8 @@ mans_status decompress_impl(mans_workspace* ws, mans_dtype dtype, mans_layout la
   if (dtype == MANS_U16) m += merged_pad(adm_u16_header_bytes(n_elems, (int)layout));
   if (unmap_only) {
     if (in_size > ws->merged_cap) return MANS_ERR_TOO_LARGE;
-    import_merged_kernel<<<copy_grid(ws->cfg, in_size), 256, 0, s>>>((const uint8_t*)d_in, m,
-                                                                      in_size, ws->ctrl);
-    e = cudaGetLastError();
+    e = launch(import_merged_kernel, copy_grid(ws->cfg, in_size), 256, 0, s, (const uint8_t*)d_in, m,
+               in_size, ws->ctrl);
   } else {
     e = launch_ans_decode((const uint8_t*)d_in, in_size, m, ws->merged_cap, ws->ctrl, -1, 1,
                           div_up_u64(n_elems + n_elems / 4, kAnsBlock),

@@ -20,6 +20,24 @@ struct NvtxRange {
   NvtxRange& operator=(const NvtxRange&) = delete;
 };
 
+// Launch a kernel that opens with kernel_begin() (mans_device.cuh): it may be
+// set up while the stream's previous kernel still runs.
+template <typename... P, typename... A>
+inline cudaError_t launch(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+                          cudaStream_t s, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 struct LaunchCfg {
   int sms = 148;        // multiprocessors of the device
   int enc_ctas = 0;     // resident CTAs per SM of the encode kernel (shared-memory staging)
