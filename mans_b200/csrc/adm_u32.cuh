@@ -305,6 +305,31 @@ __device__ __forceinline__ void unmap32_group(const uint8_t* __restrict__ M, uin
     return;
   }
   const uint8_t* src = M + rec_base + goff;
+  // A full group with 16 record bytes in every lane holds one code byte per
+  // element and nothing else (half of the detector frames' groups): each lane
+  // reads its own, about 200 instructions instead of 900 (1 GiB of frames: 0.555
+  // -> 0.455 ms; data without such groups keeps its time).
+  if (__all_sync(0xffffffffu, len == 16 && cnt == 16)) {
+    const uint2* own = reinterpret_cast<const uint2*>(src + 16 * lane);
+    const uint2 a = __ldg(own), b = __ldg(own + 1);
+    const uint32_t w[4] = {a.x, a.y, b.x, b.y};
+    uint32_t odd = 0;  // bytes that are no code here: 0, 254, 255
+    uint4* dst = reinterpret_cast<uint4*>(out + ls);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t hi = ~(w[q] | 0x01010101u);  // a zero byte for 254 and 255
+      odd |= (((w[q] - 0x01010101u) & ~w[q]) | ((hi - 0x01010101u) & ~hi)) & 0x80808080u;
+      uint32_t r[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t code = __byte_perm(w[q], 0u, 0x4440u | i);
+        r[i] = (code & 1u) ? c - (code >> 1) : c + (code >> 1);
+      }
+      dst[q] = make_uint4(r[0], r[1], r[2], r[3]);
+    }
+    if (__any_sync(0xffffffffu, odd != 0) && lane == 0) report(sink, MANS_ERR_CORRUPT, grp);
+    return;
+  }
   __syncwarp();
   warp_load_phase(stage, src, gtot, lane);
   __syncwarp();

@@ -118,3 +118,37 @@ def test_batch_decoder_chunks(oracle, big):
         assert big_in is None or torch.equal(outs[-1], big_in)
     finally:
         b.close()
+
+
+@pytest.mark.parametrize("n", [512, 511, 512 * 37, 512 * 37 + 300])
+@pytest.mark.parametrize("spread", [0, 126, 127, 300])
+def test_u32_groups_of_one_byte_codes(ws, oracle, n, spread):
+    """Groups at and around the limit of one code byte per element, high and
+    low centers, mixed with groups that need more."""
+    import torch
+    rng = np.random.default_rng(n + spread)
+    x = np.empty(n, np.uint32)
+    for g in range(0, n, 512):
+        m = min(512, n - g)
+        c = int(rng.choice([0, 130, 70_000, (1 << 32) - 1 - 2 * spread]))
+        v = c + spread + rng.integers(-spread, spread + 1, m) * (rng.random(m) < 0.05)
+        x[g:g + m] = np.clip(v, 0, (1 << 32) - 1).astype(np.uint32)
+    s = mb.compress(to_dev(x), 10, ws=ws)
+    np.testing.assert_array_equal(to_host(s), oracle.compress(x, 10))
+    np.testing.assert_array_equal(to_host(mb.decompress(s, n, torch.uint32, ws=ws), np.uint32), x)
+
+
+@pytest.mark.parametrize("byte", [0, 254, 255])
+def test_u32_one_byte_group_with_a_bad_code(ws, byte):
+    """A byte that is no code in a group of 16-byte records is reported."""
+    import torch
+    x = np.full(1024, 1000, np.uint32)
+    m = to_host(mb.adm_map(to_dev(x), ws=ws)).copy()
+    assert m.size == 80 + 1024
+    for at in (80, 80 + 511, 80 + 700):
+        bad = m.copy()
+        bad[at] = byte
+        with pytest.raises(mb.MansError) as e:
+            mb.adm_unmap(to_dev(bad), x.size, torch.uint32, ws=ws)
+        assert e.value.code == 10  # MANS_ERR_CORRUPT
+    np.testing.assert_array_equal(to_host(mb.adm_unmap(to_dev(m), x.size, torch.uint32, ws=ws), np.uint32), x)
