@@ -120,6 +120,56 @@ __device__ __forceinline__ void map32_stage(const uint32_t* __restrict__ in, uin
   if (fill) *reinterpret_cast<uint64_t*>(rec + wpos) = lo | (~0ull << (8 * fill));
 }
 
+// Stage a group's records: each lane's elements are measured, measured(bytes)
+// is called with the group's record bytes (returned too), and the lane's
+// record is staged. v, c, cnt: the lane's values, the center, its valid values
+// (in + ls on); lens: the group's 32 record lengths in M.
+template <typename Measured>
+__device__ __forceinline__ uint32_t map32_records(const uint32_t* __restrict__ in, uint64_t ls,
+                                                  const uint32_t (&v)[16], uint32_t c, int cnt,
+                                                  uint8_t* lens, uint32_t* hist, uint8_t* stage,
+                                                  int lane, Measured measured) {
+  // each element once: bytes (k or 5), code byte, escape flag
+  uint32_t nbp[2] = {0, 0};      // 4-bit byte counts
+  uint32_t codes[4] = {0, 0, 0, 0};
+  uint32_t escm = 0, rlen = 0;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    uint32_t nb, code;
+    bool esc;
+    adm_elem_u32(v[i], c, nb, code, esc);
+    nb = i < cnt ? nb : 0u;
+    nbp[i >> 3] |= nb << ((i & 7) * 4);
+    codes[i >> 2] |= code << ((i & 3) * 8);
+    escm |= (esc && i < cnt) ? (1u << i) : 0u;
+    rlen += nb;
+  }
+  const uint32_t padded = (rlen + 7) & ~7u;
+  uint32_t incl = padded;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  const uint32_t loff = incl - padded;
+  const uint32_t gtot = __shfl_sync(0xffffffffu, incl, 31);
+
+  measured(gtot);
+  if (cnt == 16) map32_stage<true>(in, ls, nbp, codes, escm, hist, stage + loff);
+  else map32_stage<false>(in, ls, nbp, codes, escm, hist, stage + loff);
+  {
+    // zero bytes: all bytes that are not codes, escapes or padding
+    const uint32_t nesc = __popc(escm);
+    const uint32_t ncode = (uint32_t)cnt - nesc;
+    const uint32_t zeros = rlen - ncode - 5 * nesc;
+    if (zeros) atomicAdd(&hist[0], zeros);
+    if (padded > rlen) atomicAdd(&hist[255], padded - rlen);
+  }
+  lens[lane] = (uint8_t)(padded >> 3);
+  atomicAdd(&hist[padded >> 3], 1u);
+  return gtot;
+}
+
 // Map group `grp` of one buffer (one warp). flags: the buffer's per-group
 // look-back flags; msize_out: written by the buffer's last group; hist: the
 // warp's shared histogram; stage: the warp's kGroupRecMax + 16 byte stage.
@@ -146,46 +196,12 @@ __device__ __forceinline__ void map32_group(const uint32_t* __restrict__ in, uin
   const uint32_t gcnt = (uint32_t)min_u64(kAdmGroup, n - gs);
   const uint32_t c = (uint32_t)(gcnt == kAdmGroup ? (lsum >> 9) : lsum / gcnt);
 
-  // each element once: bytes (k or 5), code byte, escape flag
-  uint32_t nbp[2] = {0, 0};      // 4-bit byte counts
-  uint32_t codes[4] = {0, 0, 0, 0};
-  uint32_t escm = 0, rlen = 0;
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    uint32_t nb, code;
-    bool esc;
-    adm_elem_u32(v[i], c, nb, code, esc);
-    nb = i < cnt ? nb : 0u;
-    nbp[i >> 3] |= nb << ((i & 7) * 4);
-    codes[i >> 2] |= code << ((i & 3) * 8);
-    escm |= (esc && i < cnt) ? (1u << i) : 0u;
-    rlen += nb;
-  }
-  const uint32_t padded = (rlen + 7) & ~7u;
-  uint32_t incl = padded;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
-  }
-  const uint32_t loff = incl - padded;
-  const uint32_t gtot = __shfl_sync(0xffffffffu, incl, 31);
-
-  // publish the group's aggregate now; the prefix is read after staging
-  if (lane == 0) st_flag(&flags[grp], make_flag(grp == 0 ? kFlagIncl : kFlagAgg, epoch, gtot));
-
-  if (cnt == 16) map32_stage<true>(in, ls, nbp, codes, escm, hist, stage + loff);
-  else map32_stage<false>(in, ls, nbp, codes, escm, hist, stage + loff);
-  {
-    // zero bytes: all bytes that are not codes, escapes or padding
-    const uint32_t nesc = __popc(escm);
-    const uint32_t ncode = (uint32_t)cnt - nesc;
-    const uint32_t zeros = rlen - ncode - 5 * nesc;
-    if (zeros) atomicAdd(&hist[0], zeros);
-    if (padded > rlen) atomicAdd(&hist[255], padded - rlen);
-  }
-  M[8 * g + 32ull * grp + lane] = (uint8_t)(padded >> 3);
-  atomicAdd(&hist[padded >> 3], 1u);
+  // publish the group's aggregate as soon as it is known; the prefix is read
+  // after staging
+  const uint32_t gtot = map32_records(in, ls, v, c, cnt, M + 8 * g + 32ull * grp, hist, stage, lane,
+                                      [&](uint32_t bytes) {
+    if (lane == 0) st_flag(&flags[grp], make_flag(grp == 0 ? kFlagIncl : kFlagAgg, epoch, bytes));
+  });
 
   // group record offset (predecessors have had the staging time to finish)
   uint32_t goff = 0;
@@ -218,6 +234,68 @@ __device__ __forceinline__ void map32_group(const uint32_t* __restrict__ in, uin
     for (uint32_t i = lane; i < gtot / 8; i += 32) dst[i] = src[i];
   }
   __syncwarp();
+}
+
+// Map group `grp` with its records in a slot of its own (kGroupRecMax bytes,
+// 16-byte aligned) instead of at their offset: no look-back. The offset field
+// of M holds the group's record bytes until the scan replaces it
+// (adm_u32_scan_kernel), which also counts the field's bytes.
+__device__ __forceinline__ void map32_slot(const uint32_t* __restrict__ in, uint64_t n,
+                                           uint8_t* __restrict__ M, uint8_t* __restrict__ slot,
+                                           uint64_t grp, uint32_t* hist, uint8_t* stage, int lane) {
+  const uint64_t g = div_up_u64(n, kAdmGroup);
+  uint32_t v[16];
+  load_lane_u32(in, n, grp, lane, v);
+  const uint64_t gs = grp * kAdmGroup;
+  const uint64_t ls = gs + (uint64_t)lane * kAdmChunk;
+  const int cnt = ls >= n ? 0 : (int)min_u64(16, n - ls);
+  unsigned long long lsum = 0;
+  uint32_t vmin = v[0], vmax = v[0];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    lsum += v[i];
+    vmin = min(vmin, v[i]);
+    vmax = max(vmax, v[i]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+  vmin = __reduce_min_sync(0xffffffffu, vmin);
+  vmax = __reduce_max_sync(0xffffffffu, vmax);
+  const uint32_t gcnt = (uint32_t)min_u64(kAdmGroup, n - gs);
+  const uint32_t c = (uint32_t)(gcnt == kAdmGroup ? (lsum >> 9) : lsum / gcnt);
+  uint8_t* const lens = M + 8 * g + 32 * grp;
+  uint32_t bytes;
+  if (gcnt == kAdmGroup && vmax - c <= kAdmStep && c - vmin <= kAdmStep) {
+    // all values within 126 of the center: one code byte per element, 16 per
+    // lane, no padding (half of the detector frames' groups)
+    bytes = kAdmGroup;
+    uint32_t w[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      uint32_t cb[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int d = (int)(v[4 * q + i] - c);
+        cb[i] = 2u * (uint32_t)abs(d) + (d <= 0 ? 1u : 0u);
+        atomicAdd(&hist[cb[i]], 1u);
+      }
+      w[q] = __byte_perm(__byte_perm(cb[0], cb[1], 0x1140u), __byte_perm(cb[2], cb[3], 0x1140u), 0x5410u);
+    }
+    reinterpret_cast<uint4*>(slot)[lane] = make_uint4(w[0], w[1], w[2], w[3]);
+    lens[lane] = 2;
+    if (lane == 0) atomicAdd(&hist[2], 32u);
+  } else {
+    bytes = map32_records(in, ls, v, c, cnt, lens, hist, stage, lane, [](uint32_t) {});
+    __syncwarp();
+    const uint4* src = reinterpret_cast<const uint4*>(stage);
+    for (uint32_t i = lane; i < (bytes + 15) / 16; i += 32) reinterpret_cast<uint4*>(slot)[i] = src[i];
+    __syncwarp();
+  }
+  if (lane == 0) {
+    reinterpret_cast<uint32_t*>(M)[grp] = bytes;
+    reinterpret_cast<uint32_t*>(M + 4 * g)[grp] = c;
+  }
+  if (lane < 4) atomicAdd(&hist[(c >> (8 * lane)) & 0xffu], 1u);
 }
 
 // ------------------------------------------------------------------------

@@ -104,11 +104,12 @@ __device__ __forceinline__ void encode_done(Ctrl* ctrl, uint32_t epoch) {
   }
 }
 
-template <int kP>
+// kGather: the input's records lie in slots (enc_gather).
+template <int kP, bool kGather>
 __global__ __launch_bounds__(kEncMaxThreads, 1) void ans_encode_slots_kernel(
     const uint8_t* __restrict__ in, uint8_t* __restrict__ out, uint64_t out_cap,
     unsigned long long* out_size64, uint32_t* out_size32, Ctrl* ctrl, unsigned long long* flags,
-    uint8_t* __restrict__ slots) {
+    uint8_t* __restrict__ slots, const AnsGather gather) {
   kernel_begin();
   extern __shared__ __align__(16) uint8_t smem_raw[];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -140,13 +141,14 @@ __global__ __launch_bounds__(kEncMaxThreads, 1) void ans_encode_slots_kernel(
   while (!failed) {
     const uint32_t b = warp_claim(&ctrl->tile_counter[1], lane);
     if (b >= nb) break;
-    if (lane == 0 && (uint64_t)b + ahead < nb) {
+    if (!kGather && lane == 0 && (uint64_t)b + ahead < nb) {
       const uint64_t s1 = ((uint64_t)b + ahead) * kAnsBlock;
       prefetch_l2(in + s1, (uint32_t)min_u64(kAnsBlock, n - s1));
     }
     uint16_t* const sout = slot0 + cur * (kEncSlotBytes / 2);
     uint32_t x;
-    const uint32_t nw = encode_words_rep<kP>(in, n, b, smem_raw, sw, parity, sout, sink, lane, x);
+    const uint32_t nw = encode_words_rep<kP, kGather>(in, n, b, smem_raw, sw, parity, sout, sink,
+                                                      lane, x, gather, (uint64_t)b + ahead);
     if (lane == 0)
       st_flag(&flags[b], make_flag(b == 0 ? kFlagIncl : kFlagAgg, epoch, (nw + 7) & ~7u));
     if (pend.b != 0xffffffffu)
@@ -342,7 +344,9 @@ static int occupancy(const void* fn, int threads, size_t smem) {
 }
 
 void init_ans_launch_cfg(LaunchCfg& cfg) {
-  for (auto* k : {ans_encode_slots_kernel<9>, ans_encode_slots_kernel<10>, ans_encode_slots_kernel<11>})
+  for (auto* k : {ans_encode_slots_kernel<9, false>, ans_encode_slots_kernel<10, false>,
+                  ans_encode_slots_kernel<11, false>, ans_encode_slots_kernel<9, true>,
+                  ans_encode_slots_kernel<10, true>, ans_encode_slots_kernel<11, true>})
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)enc_smem_bytes(kEncMaxWarps));
   cudaFuncSetAttribute(ans_encode_shared_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -371,7 +375,7 @@ cudaError_t launch_ans_encode(const uint8_t* in, uint8_t* out, uint64_t out_cap,
                               unsigned long long* out_size64, uint32_t* out_size32, Ctrl* ctrl,
                               unsigned long long* flags, int prob_bits, uint64_t likely_blocks,
                               uint64_t max_blocks, const LaunchCfg& cfg, cudaStream_t s,
-                              uint8_t* slots) {
+                              uint8_t* slots, const AnsGather* gather) {
   if (slots) {
     // one CTA per SM with as many warps as spread the blocks evenly
     uint64_t warps = div_up_u64(likely_blocks, (uint64_t)cfg.sms);
@@ -379,11 +383,15 @@ cudaError_t launch_ans_encode(const uint8_t* in, uint8_t* out, uint64_t out_cap,
     const uint64_t want = div_up_u64(max_blocks, warps);
     const unsigned grid =
         (unsigned)(want < 1 ? 1 : (want < (uint64_t)cfg.sms ? want : (uint64_t)cfg.sms));
-    auto* k = prob_bits == 9    ? ans_encode_slots_kernel<9>
-              : prob_bits == 10 ? ans_encode_slots_kernel<10>
-                                : ans_encode_slots_kernel<11>;
+    auto* k = prob_bits == 9    ? ans_encode_slots_kernel<9, false>
+              : prob_bits == 10 ? ans_encode_slots_kernel<10, false>
+                                : ans_encode_slots_kernel<11, false>;
+    if (gather)
+      k = prob_bits == 9    ? ans_encode_slots_kernel<9, true>
+          : prob_bits == 10 ? ans_encode_slots_kernel<10, true>
+                            : ans_encode_slots_kernel<11, true>;
     return launch(k, grid, (unsigned)warps * 32, enc_smem_bytes((int)warps), s, in, out, out_cap,
-                  out_size64, out_size32, ctrl, flags, slots);
+                  out_size64, out_size32, ctrl, flags, slots, gather ? *gather : AnsGather{});
   } else {
     const uint64_t want = div_up_u64(max_blocks, kEncWarps);
     const uint64_t cap = (uint64_t)cfg.sms * cfg.enc_ctas;

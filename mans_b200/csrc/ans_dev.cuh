@@ -7,6 +7,7 @@
 #pragma once
 
 #include "ans_table.cuh"
+#include "mans_internal.h"
 #include "smem_io.cuh"
 
 namespace mans {
@@ -169,6 +170,17 @@ __device__ __forceinline__ uint32_t encode_words(const uint8_t* __restrict__ in,
   return nw;
 }
 
+// ---- asynchronous copies global -> shared ----
+__device__ __forceinline__ void cp_async16(uint32_t smem, const void* g) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(g) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t smem, const void* g) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem), "l"(g) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 // ---- encode with replicated tables (word slots in global memory) ----
 // The step's integer instructions bound the coder (the ALU pipe issues at half
 // rate), and shared-memory wavefronts come next. 16-byte entries need the
@@ -296,22 +308,81 @@ __device__ __forceinline__ uint32_t encode_staged_rep(const uint8_t* syms, uint3
   return done / 2 + rem;
 }
 
+// Stage block [b0, b1) of a mapped uint32 buffer whose records lie in slots
+// (AnsGather): all parts begin and end on 8-byte boundaries. A full group has
+// 512 record bytes at least, so a block holds parts of ten groups at most (and
+// of one short last group). Also prefetches the records of block `later` into
+// L2 (past the last block: nothing).
+__device__ __forceinline__ void enc_gather(const uint8_t* __restrict__ in, uint64_t n, uint32_t b,
+                                           uint64_t later, const AnsGather& src, uint8_t* stage,
+                                           int lane) {
+  const uint64_t b0 = (uint64_t)b * kAnsBlock, b1 = min_u64(b0 + kAnsBlock, n);
+  const uint64_t rb = 40 * src.groups;
+  const uint32_t* off = reinterpret_cast<const uint32_t*>(in);
+  const uint32_t total = (uint32_t)(n - rb);
+  const uint64_t l0 = later * kAnsBlock, l1 = min_u64(l0 + kAnsBlock, n);
+  const bool ahead = l0 < n && l1 > rb;
+  const uint32_t f = b1 > rb ? src.first_group[b] : 0u;
+  const uint32_t lf = ahead ? src.first_group[later] : 0u;
+  auto offset = [&](uint64_t k) { return k < src.groups ? off[k] : total; };
+  const uint32_t o = offset((uint64_t)f + lane);
+  const uint32_t lo = offset((uint64_t)lf + lane), lo1 = __shfl_down_sync(0xffffffffu, lo, 1);
+  if (ahead && lane < 12 && lo < lo1 && rb + lo < l1)
+    prefetch_l2(src.slots + ((uint64_t)lf + lane) * 4096, lo1 - lo);
+  const uint32_t dst = smem_addr(stage);
+  if (b0 < rb) {
+    const uint32_t h = (uint32_t)(min_u64(b1, rb) - b0);
+    for (uint32_t i = 8 * lane; i < h; i += 256) cp_async8(dst + i, in + b0 + i);
+  }
+  if (b1 > rb) {
+    // lane k: its group's part of record bytes [r0, r1), in the slots and in
+    // the stage
+    const uint32_t r0 = (uint32_t)(b0 > rb ? b0 - rb : 0), r1 = (uint32_t)(b1 - rb);
+    const uint32_t o1 = __shfl_down_sync(0xffffffffu, o, 1);
+    const uint32_t p0 = max(o, r0), len = min(o1, r1) - p0;
+    const uint32_t from = 4096u * lane + p0 - o;
+    const uint32_t to = dst + (uint32_t)(b0 > rb ? 0 : rb - b0) + p0 - r0;
+    const uint32_t parts = __popc(__ballot_sync(0xffffffffu, lane < 31 && o < r1));
+    const uint8_t* const g = src.slots + (uint64_t)f * 4096 + 8 * lane;
+    for (uint32_t k = 0; k < parts; ++k) {
+      const uint32_t n8 = __shfl_sync(0xffffffffu, len, k);
+      const uint8_t* p = g + __shfl_sync(0xffffffffu, from, k);
+      uint32_t q = __shfl_sync(0xffffffffu, to, k) + 8 * lane;
+      for (uint32_t i = 8 * lane; i < n8; i += 1024, p += 1024, q += 1024) {
+        cp_async8(q, p);
+#pragma unroll
+        for (uint32_t u = 256; u < 1024; u += 256)
+          if (i + u < n8) cp_async8(q + u, p + u);
+      }
+    }
+  }
+  cp_async_wait_all();
+}
+
 // encode_words for the replicated table: block b of one buffer (one warp).
-template <int kP>
+// kGather: the block's bytes come from slots (src), and block `later` is
+// prefetched.
+template <int kP, bool kGather>
 __device__ __forceinline__ uint32_t encode_words_rep(const uint8_t* __restrict__ in, uint64_t n,
                                                      uint32_t b, const uint8_t* tab, EncWarp& sw,
                                                      uint32_t& parity, uint16_t* slot,
-                                                     const Sink& sink, int lane, uint32_t& x) {
+                                                     const Sink& sink, int lane, uint32_t& x,
+                                                     const AnsGather& src, uint64_t later) {
   const uint64_t start = (uint64_t)b * kAnsBlock;
   const uint32_t bs = (uint32_t)min_u64(kAnsBlock, n - start);
   __syncwarp();  // the previous block's reads of the stage are complete
-  if (lane == 0) {
+  if (kGather) {
+    enc_gather(in, n, b, later, src, sw.in, lane);
+    __syncwarp();
+  } else if (lane == 0) {
     const uintptr_t a0 = reinterpret_cast<uintptr_t>(in + start) & ~uintptr_t(15);
     const uintptr_t a1 = (reinterpret_cast<uintptr_t>(in + start) + bs + 15) & ~uintptr_t(15);
     bulk_load(sw.in, reinterpret_cast<const void*>(a0), (uint32_t)(a1 - a0), &sw.bar);
   }
-  if (!mbar_wait(&sw.bar, parity) && lane == 0) report(sink, MANS_ERR_TIMEOUT, b);
-  parity ^= 1u;
+  if (!kGather) {
+    if (!mbar_wait(&sw.bar, parity) && lane == 0) report(sink, MANS_ERR_TIMEOUT, b);
+    parity ^= 1u;
+  }
   uint32_t nw = encode_staged_rep<kP>(sw.in + phase16(in + start) + lane, bs, tab, sw.words,
                                       reinterpret_cast<uint8_t*>(slot), lane, x);
   if (nw > kAnsMaxBlockWords) {  // see encode_words
@@ -527,14 +598,6 @@ struct DecWhole {
   alignas(16) uint16_t words[kEncOutWords];
   alignas(16) uint8_t out[kDecChunkBytes + 16];
 };
-
-// ---- asynchronous 16-byte copies global -> shared ----
-__device__ __forceinline__ void cp_async16(uint32_t smem, const void* g) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(g) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.wait_all;" ::: "memory");
-}
 
 // Store one decoded 512-byte chunk from the warp's stage, where it sits at
 // offset ph = g & 15 (the destination's phase), to g: 16-byte stores for the

@@ -42,7 +42,9 @@ struct mans_workspace {
   uint64_t ans_flags_n = 0;
   uint8_t* merged = nullptr;  // 16-byte aligned region of merged_cap + slack bytes
   uint8_t* enc_slots = nullptr;  // per-warp word slots of the encode kernel
-  uint32_t* v12_excl = nullptr;  // group offsets of the V12 layout's unmap
+  // a word per KiB of input: group offsets of the V12 layout's unmap, first
+  // groups of the blocks of a gathered uint32 compress
+  uint32_t* group_scratch = nullptr;
   LaunchCfg cfg;
   // Opt-in kernel timing: a ring of event triples per recorded call
   // (compress: start, after mapping, after encode; decompress: start, after
@@ -165,6 +167,11 @@ unsigned copy_grid(const LaunchCfg& cfg, uint64_t n) {
   return (unsigned)(want < 1 ? 1 : (want < cap ? want : cap));
 }
 
+// From this many uint32 values on, a compress leaves the records in slots
+// (1 M values of detector frames: map and encode 49.3 us with the single-pass
+// map, 51.7 so; 4 M: 75 and 69; 2^28: 1,587 and 1,340).
+constexpr uint64_t kSplitMin = 1u << 21;
+
 bool valid_layout(mans_dtype dtype, mans_layout layout) {
   if (layout == MANS_LAYOUT_NATIVE) return true;
   return dtype == MANS_U16 && (layout == MANS_LAYOUT_V12 || layout == MANS_LAYOUT_CPUV2);
@@ -187,6 +194,8 @@ mans_status compress_impl(mans_workspace* ws, mans_dtype dtype, mans_layout layo
   cudaError_t e = cudaSuccess;
   if (dtype == MANS_U8 && in_bytes > kMaxMerged) return MANS_ERR_TOO_LARGE;
   uint8_t* m = nullptr;
+  AnsGather gather;
+  bool split = false;
   mark(ws, 0, s);
   if (dtype == MANS_U8) {
     e = launch_hist_bytes((const uint8_t*)d_in, in_bytes, ws->ctrl, precision, ws->cfg, s);
@@ -209,7 +218,13 @@ mans_status compress_impl(mans_workspace* ws, mans_dtype dtype, mans_layout layo
     // 16-byte aligned; the records (40 bytes a group on) are then 8-byte aligned
     if (adm_u32_header_bytes(n_elems) + n_elems > ws->merged_cap) return MANS_ERR_TOO_LARGE;
     m = ws->merged;
-    e = launch_adm_u32_map((const uint32_t*)d_in, n_elems, m, ws->merged_cap, ws->ctrl,
+    // Large inputs leave their records in slots for the encoder to gather, if
+    // the workspace has room for them (the default capacity does).
+    split = !map_only && n_elems >= kSplitMin && adm_u32_split_bytes(n_elems) <= ws->merged_cap;
+    if (split)
+      e = launch_adm_u32_split((const uint32_t*)d_in, n_elems, m, ws->group_scratch, ws->ctrl,
+                               ws->adm_flags, precision, ws->cfg, s, &gather);
+    else e = launch_adm_u32_map((const uint32_t*)d_in, n_elems, m, ws->merged_cap, ws->ctrl,
                            ws->adm_flags, precision, ws->cfg, s);
   }
   mark(ws, 1, s);
@@ -221,7 +236,8 @@ mans_status compress_impl(mans_workspace* ws, mans_dtype dtype, mans_layout layo
       // an element maps to one byte, and a little more
       e = launch_ans_encode(m, (uint8_t*)d_out, out_capacity, osz, nullptr, ws->ctrl,
                             ws->ans_flags, precision, div_up_u64(n_elems + n_elems / 4, kAnsBlock),
-                            div_up_u64(ws->merged_cap, kAnsBlock), ws->cfg, s, ws->enc_slots);
+                            div_up_u64(ws->merged_cap, kAnsBlock), ws->cfg, s, ws->enc_slots,
+                            split ? &gather : nullptr);
     }
   }
   mark(ws, 2, s);
@@ -266,7 +282,7 @@ mans_status decompress_impl(mans_workspace* ws, mans_dtype dtype, mans_layout la
   if (e == cudaSuccess) {
     if (dtype == MANS_U16)
       e = launch_adm_u16_unmap(m, n_elems, (uint16_t*)d_out, ws->ctrl, ws->cfg, s, (int)layout,
-                               ws->v12_excl, ws->ans_flags);
+                               ws->group_scratch, ws->ans_flags);
     else
       e = launch_adm_u32_unmap(m, n_elems, (uint32_t*)d_out, ws->ctrl, ws->cfg, s);
   }
@@ -303,8 +319,8 @@ mans_status mans_workspace_create(mans_workspace** out, uint64_t max_input_bytes
   const uint64_t off_adm = align_up(sizeof(Ctrl), 256);
   const uint64_t off_ans = align_up(off_adm + 8 * ws->adm_flags_n, 256);
   const uint64_t off_slots = align_up(off_ans + 8 * ws->ans_flags_n, 256);
-  const uint64_t off_v12 = align_up(off_slots + ans_encode_slot_bytes(ws->cfg), 256);
-  const uint64_t off_m = align_up(off_v12 + 4 * ws->adm_flags_n, 256);
+  const uint64_t off_group = align_up(off_slots + ans_encode_slot_bytes(ws->cfg), 256);
+  const uint64_t off_m = align_up(off_group + 4 * ws->adm_flags_n, 256);
   ws->bytes = align_up(off_m + merged_capacity + kSlack, 256);
   if (cudaMalloc(&ws->base, ws->bytes) != cudaSuccess) {
     cudaGetLastError();
@@ -320,7 +336,7 @@ mans_status mans_workspace_create(mans_workspace** out, uint64_t max_input_bytes
   ws->adm_flags = reinterpret_cast<unsigned long long*>(ws->base + off_adm);
   ws->ans_flags = reinterpret_cast<unsigned long long*>(ws->base + off_ans);
   ws->enc_slots = ws->base + off_slots;
-  ws->v12_excl = reinterpret_cast<uint32_t*>(ws->base + off_v12);
+  ws->group_scratch = reinterpret_cast<uint32_t*>(ws->base + off_group);
   ws->merged = ws->base + off_m;
   *out = ws;
   return MANS_OK;

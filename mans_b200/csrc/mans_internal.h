@@ -43,12 +43,22 @@ struct LaunchCfg {
   int enc_ctas = 0;     // resident CTAs per SM of the encode kernel (shared-memory staging)
   int map_ctas = 0;     // resident CTAs per SM of the ADM map kernels
   int map32_ctas = 0;   // resident CTAs per SM of the uint32 ADM map kernel
+  int split32_ctas = 0; // ... of the uint32 map that leaves records in slots
   int unmap32_ctas = 0; // resident CTAs per SM of the uint32 ADM unmap kernel
   int hist_ctas = 0;    // resident CTAs per SM of the byte histogram kernel
 };
 
 // Query occupancy once per device.
 void init_launch_cfg(LaunchCfg& cfg, int device);
+
+// A mapped uint32 buffer whose records lie in slots: byte 40 * groups + r of
+// the buffer (r in group k, whose records start at offset o_k = the buffer's
+// 32-bit word k) is byte r - o_k of slot k, 4,096 bytes each.
+struct AnsGather {
+  const uint8_t* slots = nullptr;
+  const uint32_t* first_group = nullptr;  // per 4 KiB block: the group of its first record byte
+  uint64_t groups = 0;
+};
 
 // ---- rANS over bytes (ans_codec.cu) ----
 // Histogram of n raw bytes + normalisation into ctrl (table, pdf, merged_size = n).
@@ -63,7 +73,8 @@ cudaError_t launch_ans_encode(const uint8_t* in, uint8_t* out, uint64_t out_cap,
                               unsigned long long* out_size64, uint32_t* out_size32, Ctrl* ctrl,
                               unsigned long long* flags, int prob_bits, uint64_t likely_blocks,
                               uint64_t max_blocks, const LaunchCfg& cfg, cudaStream_t s,
-                              uint8_t* slots);
+                              uint8_t* slots, const AnsGather* gather = nullptr);
+// gather (with slots): the input's records lie in slots of their own.
 uint64_t ans_encode_slot_bytes(const LaunchCfg& cfg);
 // Decode the stream at `in` into `out` (at most out_cap bytes). expect_p < 0
 // accepts any valid precision. record != 0 stores the decoded size in ctrl.
@@ -90,6 +101,13 @@ cudaError_t launch_adm_u16_unmap(const uint8_t* m, uint64_t n, uint16_t* out, Ct
 cudaError_t launch_adm_u32_map(const uint32_t* in, uint64_t n, uint8_t* m, uint64_t m_cap,
                                Ctrl* ctrl, unsigned long long* flags, int prob_bits,
                                const LaunchCfg& cfg, cudaStream_t s);
+// The same for launch_ans_encode with `gather`, which is filled: records in
+// slots behind the header (adm_u32_split_bytes(n) bytes at m in all).
+// first_group: one entry per 4 KiB block of the mapped buffer.
+uint64_t adm_u32_split_bytes(uint64_t n);
+cudaError_t launch_adm_u32_split(const uint32_t* in, uint64_t n, uint8_t* m, uint32_t* first_group,
+                                 Ctrl* ctrl, unsigned long long* flags, int prob_bits,
+                                 const LaunchCfg& cfg, cudaStream_t s, AnsGather* gather);
 cudaError_t launch_adm_u32_unmap(const uint8_t* m, uint64_t n, uint32_t* out, Ctrl* ctrl,
                                  const LaunchCfg& cfg, cudaStream_t s);
 

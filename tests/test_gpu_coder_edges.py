@@ -152,3 +152,28 @@ def test_u32_one_byte_group_with_a_bad_code(ws, byte):
             mb.adm_unmap(to_dev(bad), x.size, torch.uint32, ws=ws)
         assert e.value.code == 10  # MANS_ERR_CORRUPT
     np.testing.assert_array_equal(to_host(mb.adm_unmap(to_dev(m), x.size, torch.uint32, ws=ws), np.uint32), x)
+
+
+@pytest.mark.parametrize("kind", ["detector", "quant", "near", "wide"])
+@pytest.mark.parametrize("n", [(1 << 21) - 1, 1 << 21, 4608 * 512, 4608 * 512 + 1, (1 << 22) + 777])
+def test_u32_records_gathered_by_the_encoder(oracle, n, kind):
+    """The two ways a uint32 compress can go, at their border and where the
+    records begin on a block's start (4,608 groups); a workspace without room
+    for the slots takes the other way, to the same bytes."""
+    import torch
+    rng = np.random.default_rng(n)
+    x = {"detector": lambda: W.detector_u32(n, 1), "quant": lambda: W.quant_u32(n, 2),
+         "near": lambda: rng.integers(0, 90, n).astype(np.uint32),
+         "wide": lambda: rng.integers(0, 1 << 32, n, dtype=np.uint64).astype(np.uint32)}[kind]()
+    ref = oracle.compress(x, 10)
+    d = to_dev(x)
+    groups = -(-n // 512)
+    for merged in (0, 4000 * groups if kind != "wide" else 0):
+        w = mb.Workspace(4 * n, merged)
+        try:
+            s = mb.compress(d, 10, ws=w)
+            np.testing.assert_array_equal(to_host(s), ref)
+            y = mb.decompress(s, n, torch.uint32, ws=w)
+        finally:
+            w.close()
+        np.testing.assert_array_equal(to_host(y, np.uint32), x)
