@@ -177,3 +177,19 @@ def test_u32_records_gathered_by_the_encoder(oracle, n, kind):
         finally:
             w.close()
         np.testing.assert_array_equal(to_host(y, np.uint32), x)
+
+
+@pytest.mark.parametrize("b", [40, 160, 280, 420, 800])
+@pytest.mark.parametrize("layout", [0, 1, 2])
+def test_u16_streams_around_their_word_limits(ws, oracle, b, layout):
+    """Lane streams whose halves stay below, pass 32 bits and whose sum passes
+    64; ragged end."""
+    import torch
+    n = 100_003
+    rng = np.random.default_rng(b)
+    scale = np.repeat(rng.choice([0.05, 1.0], -(-n // 8)), 8)[:n]  # per eight elements
+    x = np.clip(np.round(30000 + rng.laplace(0, 1, n) * b * scale), 0, 65535).astype(np.uint16)
+    s = mb.compress(to_dev(x), 10, ws=ws, layout=layout)
+    np.testing.assert_array_equal(to_host(s), oracle.compress(x, 10, layout))
+    y = mb.decompress(s, n, torch.uint16, ws=ws, layout=layout)
+    np.testing.assert_array_equal(to_host(y, np.uint16), x)
