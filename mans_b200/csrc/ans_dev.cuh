@@ -213,9 +213,14 @@ inline size_t enc_smem_bytes(int warps) { return kEncTableBytes + (size_t)warps 
 // Fill the table from 256 packed entries (all threads of the CTA; the caller
 // synchronises). Rotated, so that the lanes of a store spread over the banks.
 __device__ __forceinline__ void enc_fill_table(uint8_t* tab, const uint2* __restrict__ enc, int p) {
-  for (uint32_t i = threadIdx.x; i < kAnsSyms * 8; i += blockDim.x) {
-    const uint32_t sym = i & 255u, c = (i >> 8) + sym;
-    *reinterpret_cast<EncEntry4*>(tab + 128 * sym + 16 * (c & 7)) = expand_enc_entry(enc[sym], p);
+  // each entry is loaded once (a load per copy cost a small input 16 round trips
+  // to L2, one after the other)
+#pragma unroll 2
+  for (uint32_t sym = threadIdx.x; sym < kAnsSyms; sym += blockDim.x) {
+    const EncEntry4 e = expand_enc_entry(enc[sym], p);
+#pragma unroll
+    for (uint32_t c = 0; c < 8; ++c)
+      *reinterpret_cast<EncEntry4*>(tab + 128 * sym + 16 * ((c + sym) & 7)) = e;
   }
 }
 

@@ -50,7 +50,7 @@ __host__ __device__ inline uint2 make_enc_entry(uint32_t pdf, uint32_t cdf, int 
 // Writes pdf[256] and the encoder table enc[256]. total == 0 gives all zeros.
 __device__ inline void normalize_cta(const uint32_t* __restrict__ hist, uint32_t total, int p,
                                      uint32_t* __restrict__ pdf_out, uint2* __restrict__ enc_out) {
-  __shared__ uint32_t s_key[kAnsSyms];
+  __shared__ __align__(16) uint32_t s_key[kAnsSyms];
   __shared__ uint32_t s_q[kAnsSyms];
   __shared__ int s_order[kAnsSyms];
   __shared__ int s_red[8];
@@ -73,14 +73,21 @@ __device__ inline void normalize_cta(const uint32_t* __restrict__ hist, uint32_t
   int sum = 0;
 #pragma unroll
   for (int w = 0; w < 8; ++w) sum += s_red[w];
-  uint32_t key = (q << 16) | (uint32_t)t;
-  int rank = 0;
-  for (int u = 0; u < kAnsSyms; ++u) rank += s_key[u] > key;
-  s_order[rank] = t;
+  const uint32_t key = (q << 16) | (uint32_t)t;
   s_q[t] = q;
+  int diff = (int)(1u << p) - sum;
+  if (total > 0 && diff < 0) {  // the ranks matter only here
+    int rank = 0;
+    const uint4* keys = reinterpret_cast<const uint4*>(s_key);
+#pragma unroll 8
+    for (int u = 0; u < kAnsSyms / 4; ++u) {
+      const uint4 k = keys[u];
+      rank += (k.x > key) + (k.y > key) + (k.z > key) + (k.w > key);
+    }
+    s_order[rank] = t;
+  }
   __syncthreads();
 
-  int diff = (int)(1u << p) - sum;
   if (total > 0 && diff > 0) {
     while (diff > 0) {
       int it = diff < kAnsSyms ? diff : kAnsSyms;
