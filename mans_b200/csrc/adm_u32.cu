@@ -68,7 +68,9 @@ __global__ __launch_bounds__(kUnmap32Threads) void adm_u32_unmap_kernel(
 // single-pass map above spends its time waiting: a group's look-back needs
 // every earlier group's length (23% of it by itself), and making the groups
 // cheaper does not shorten that chain. 1 GiB of detector frames: map 0.945 ->
-// 0.631 ms (scan included, about 12 us), encode 0.642 -> 0.708 for the gathering.
+// 0.626 ms (scan included, about 15 us), encode 0.642 -> 0.708 for the gathering.
+// Data without groups of one-byte codes lose what those gain elsewhere (1 GiB of
+// Laplace codes: 1.102 + 0.740 -> 1.138 + 0.816 ms); the host cannot tell.
 // ------------------------------------------------------------------------
 __global__ __launch_bounds__(kMap32Threads) void adm_u32_split_kernel(
     const uint32_t* __restrict__ in, uint64_t n, uint8_t* __restrict__ M,

@@ -250,24 +250,28 @@ __device__ __forceinline__ void map32_slot(const uint32_t* __restrict__ in, uint
   const uint64_t ls = gs + (uint64_t)lane * kAdmChunk;
   const int cnt = ls >= n ? 0 : (int)min_u64(16, n - ls);
   unsigned long long lsum = 0;
-  uint32_t vmin = v[0], vmax = v[0];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    lsum += v[i];
-    vmin = min(vmin, v[i]);
-    vmax = max(vmax, v[i]);
-  }
+  for (int i = 0; i < 16; ++i) lsum += v[i];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-  vmin = __reduce_min_sync(0xffffffffu, vmin);
-  vmax = __reduce_max_sync(0xffffffffu, vmax);
   const uint32_t gcnt = (uint32_t)min_u64(kAdmGroup, n - gs);
   const uint32_t c = (uint32_t)(gcnt == kAdmGroup ? (lsum >> 9) : lsum / gcnt);
+  // all values within 126 of the center? [lo, hi] without wrapping; the lanes'
+  // first elements rule most other groups out
+  const uint32_t lo = c > kAdmStep ? c - kAdmStep : 0u;
+  const uint32_t span = (c < ~0u - kAdmStep ? c + kAdmStep : ~0u) - lo;
+  bool near = gcnt == kAdmGroup && __all_sync(0xffffffffu, v[0] - lo <= span);
+  if (near) {
+    uint32_t most = 0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) most = max(most, v[i] - lo);
+    near = __all_sync(0xffffffffu, most <= span);
+  }
   uint8_t* const lens = M + 8 * g + 32 * grp;
   uint32_t bytes;
-  if (gcnt == kAdmGroup && vmax - c <= kAdmStep && c - vmin <= kAdmStep) {
-    // all values within 126 of the center: one code byte per element, 16 per
-    // lane, no padding (half of the detector frames' groups)
+  if (near) {
+    // one code byte per element, 16 per lane, no padding (half of the detector
+    // frames' groups)
     bytes = kAdmGroup;
     uint32_t w[4];
 #pragma unroll

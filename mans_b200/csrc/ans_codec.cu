@@ -3,11 +3,11 @@
 //
 // Stream layout and arithmetic are those of include/ans (GpuANSCodec.h,
 // GpuANSEncode.h, GpuANSDecode.h); the kernels are organised differently:
-//  * encode writes the final coalesced stream directly: each warp stages its
-//    block's words in shared memory, learns its word offset through a
-//    decoupled look-back over per-block flags, and stores 16-byte vectors.
-//    The reference instead writes an uncoalesced scratch (5,248-byte stride),
-//    scans with up to three kernels and copies with a fourth.
+//  * encode writes the final coalesced stream directly: each warp collects its
+//    block's words in shared memory and a slot in L2, learns its word offset
+//    through a decoupled look-back over per-block flags, and stores 16-byte
+//    vectors. The reference instead writes an uncoalesced scratch (5,248-byte
+//    stride), scans with up to three kernels and copies with a fourth.
 //  * the table is normalised by the last CTA of the histogram kernel, not by
 //    a separate launch;
 //  * decode validates the header on the device and reports a status instead
@@ -202,8 +202,8 @@ __global__ __launch_bounds__(kEncThreads) void ans_encode_shared_kernel(
 // ------------------------------------------------------------------------
 // Decode: a warp decodes a block, or two together, from the last step to the
 // first. One CTA of up to 32 warps per SM shares the replicated slot table
-// (128 KiB). What bounds it: per step 21 instructions of which 7 go to the
-// half-rate integer ALU, two population counts, and a chain of two
+// (128 KiB). What bounds it: per step 22 instructions (block overhead included)
+// of which 7 go to the half-rate integer ALU, two population counts, and a chain of two
 // shared-memory loads, a vote and a population count (about 130 cycles) that
 // only other chains can hide. The former kernel (22 instructions, 12 of them
 // ALU, table conflicts on 40% of its shared wavefronts, 32 chains per SM
