@@ -546,8 +546,11 @@ def run_mans(args):
     if rank == 0:
         peak, peak_src = hbm_peak()
         algo = {"map": U + M, "encode": M + C, "decode": C + M, "unmap": M + U}
-        names = {"map": "adm_u32_map_kernel" if elem == 4 else "adm_u16_map_kernel",
-                 "encode": "ans_encode_kernel", "decode": "ans_decode_kernel",
+        # uint32 calls of 2 M values and more map with two kernels (the second a scan)
+        split = elem == 4 and n >= 1 << 21
+        names = {"map": ("adm_u32_split_kernel+scan" if split else
+                         "adm_u32_map_kernel" if elem == 4 else "adm_u16_map_kernel"),
+                 "encode": "ans_encode_slots_kernel", "decode": "ans_decode_kernel",
                  "unmap": "adm_u32_unmap_kernel" if elem == 4 else "adm_u16_unmap_kernel"}
         dom = max(k_ms, key=lambda k: k_ms[k])
         achieved = algo[dom] / (k_ms[dom] / 1e3) / 1e9
@@ -581,7 +584,7 @@ def run_mans(args):
             "e2e_sequential": {"value": round(world * U / (e2e_seq_step_ms / 1e3) / 1e9, 3),
                                "unit": "GB/s", "ms_per_step": round(e2e_seq_step_ms, 3),
                                "mode": "one buffer at a time"},
-            "gpu_launches": 4 * args.steps,
+            "gpu_launches": (5 if split else 4) * args.steps,
             "clocks": clk.summary(),
         }
     if dist:
