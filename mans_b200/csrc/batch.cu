@@ -46,6 +46,7 @@ __device__ __forceinline__ uint32_t find_item(uint32_t it, uint32_t count, uint6
 
 // ------------------------------------------------------------------------
 __global__ void batch_begin_kernel(BatchState* states, uint32_t count, Ctrl* ctrl) {
+  kernel_begin();
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
     states[i].status = 0;
     states[i].detail = 0;
@@ -176,6 +177,7 @@ __global__ __launch_bounds__(kBThreads, kDtype == MANS_U32 ? 3 : kDtype == MANS_
                                                               unsigned long long* flags,
                                                               uint32_t* hists, uint32_t hist_items,
                                                               uint32_t prefetch_grids) {
+  kernel_begin();
   extern __shared__ __align__(16) uint8_t smem_raw[];
   __shared__ MapHist mh;
   constexpr int kSlot = 3 + (kDtype == MANS_U8 ? 0 : kDtype == MANS_U16 ? 1 : 2);
@@ -339,6 +341,7 @@ __global__ __launch_bounds__(256) void batch_plan_encode_kernel(const BatchItem*
                                                                 unsigned long long* item_flags,
                                                                 uint32_t* hists,
                                                                 uint32_t hist_items) {
+  kernel_begin();
   __shared__ uint32_t s_item;
   __shared__ uint32_t s_hist[kAnsSyms];
   __shared__ int s_last;
@@ -422,6 +425,7 @@ __global__ __launch_bounds__(kBThreads, 4) void batch_encode_kernel(const BatchI
                                                                  unsigned long long* flags,
                                                                  uint8_t* __restrict__ slots,
                                                                  uint32_t prefetch_grids) {
+  kernel_begin();
   extern __shared__ __align__(16) uint8_t smem_raw[];
   BatchEncSmem& sm = *reinterpret_cast<BatchEncSmem*>(smem_raw);
   __shared__ int s_last;
@@ -514,6 +518,7 @@ __global__ __launch_bounds__(32) void batch_plan_decode_kernel(const BatchItem* 
                                                                Ctrl* ctrl,
                                                                unsigned long long* item_flags,
                                                                uint32_t chunk_blocks) {
+  kernel_begin();
   const int lane = threadIdx.x;
   const uint32_t epoch = *((volatile uint32_t*)&ctrl->epoch);
   while (true) {
@@ -613,6 +618,7 @@ __global__ __launch_bounds__(kDThreads, 1) void batch_decode_kernel(const BatchI
                                                                     BatchState* states, uint32_t count,
                                                                     Ctrl* ctrl,
                                                                     uint32_t chunk_blocks) {
+  kernel_begin();
   extern __shared__ __align__(16) uint8_t smem_raw[];
   BatchDecSmem& sm = *reinterpret_cast<BatchDecSmem*>(smem_raw);
   __shared__ uint32_t s_incl[kAnsSyms];
@@ -721,6 +727,7 @@ __global__ __launch_bounds__(kBThreads, kDtype == MANS_U16 ? 4 : 5) void batch_u
                                                                 BatchState* states, uint32_t count,
                                                                 uint64_t total_units, Ctrl* ctrl,
                                                                 uint32_t unit_run) {
+  kernel_begin();
   extern __shared__ __align__(16) uint8_t smem_raw[];
   __shared__ int s_last;
   constexpr int kSlot = kDtype == MANS_U16 ? 2 : 6;
@@ -796,6 +803,7 @@ __global__ __launch_bounds__(kBThreads, kDtype == MANS_U16 ? 4 : 5) void batch_u
 // ------------------------------------------------------------------------
 __global__ void batch_gather_status_kernel(const BatchState* states, uint32_t count,
                                            uint32_t* status, unsigned long long* detail) {
+  kernel_begin();
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
     status[i] = states[i].status;
     detail[i] = states[i].detail;
@@ -805,8 +813,7 @@ __global__ void batch_gather_status_kernel(const BatchState* states, uint32_t co
 cudaError_t launch_batch_gather_status(const BatchDev& d, uint32_t count, uint32_t* status,
                                        unsigned long long* detail, cudaStream_t s) {
   const unsigned grid = (unsigned)((count + 255) / 256 > 0 ? (count + 255) / 256 : 1);
-  batch_gather_status_kernel<<<grid, 256, 0, s>>>(d.states, count, status, detail);
-  return cudaGetLastError();
+  return launch(batch_gather_status_kernel, grid, 256, 0, s, d.states, count, status, detail);
 }
 
 // ------------------------------------------------------------------------
@@ -877,29 +884,32 @@ static unsigned grid_of(const BatchCfg& c, int stage, uint64_t want, int extra_o
 cudaError_t launch_batch_compress(const BatchDev& d, uint32_t count, const uint64_t groups[3],
                                   uint64_t max_blocks, const BatchCfg& c, cudaStream_t s,
                                   cudaEvent_t* marks) {
+  cudaError_t e = cudaSuccess;
+  auto go = [&](auto* kernel, unsigned grid, unsigned block, size_t smem, auto... args) {
+    if (e == cudaSuccess) e = launch(kernel, grid, block, smem, s, args...);
+  };
   if (marks) cudaEventRecord(marks[0], s);
-  batch_begin_kernel<<<(count + 255) / 256 + 1, 256, 0, s>>>(d.states, count, d.ctrl);
+  go(batch_begin_kernel, (count + 255) / 256 + 1, 256, 0, d.states, count, d.ctrl);
   const int mw = c.warps[kStageMap];
   const uint32_t mpf = (uint32_t)c.prefetch[kStageMap];
   if (groups[1])
-    batch_map_kernel<MANS_U16><<<map_grid(c, 1, groups[1], c.occ_u16_map), 32 * mw, 0, s>>>(
-        d.items, d.states, count, groups[1], d.ctrl, d.group_flags, d.hists, d.hist_items, mpf);
+    go(batch_map_kernel<MANS_U16>, map_grid(c, 1, groups[1], c.occ_u16_map), 32 * mw, 0, d.items,
+       d.states, count, groups[1], d.ctrl, d.group_flags, d.hists, d.hist_items, mpf);
   if (groups[2])
-    batch_map_kernel<MANS_U32><<<map_grid(c, 2, groups[2], 0), 32 * mw, map32_smem(mw), s>>>(
-        d.items, d.states, count, groups[2], d.ctrl, d.group_flags, d.hists, d.hist_items, mpf);
+    go(batch_map_kernel<MANS_U32>, map_grid(c, 2, groups[2], 0), 32 * mw, map32_smem(mw), d.items,
+       d.states, count, groups[2], d.ctrl, d.group_flags, d.hists, d.hist_items, mpf);
   if (groups[0])
-    batch_map_kernel<MANS_U8><<<map_grid(c, 0, groups[0], c.occ_u8_map), 32 * mw, 0, s>>>(
-        d.items, d.states, count, groups[0], d.ctrl, d.group_flags, d.hists, d.hist_items, mpf);
+    go(batch_map_kernel<MANS_U8>, map_grid(c, 0, groups[0], c.occ_u8_map), 32 * mw, 0, d.items,
+       d.states, count, groups[0], d.ctrl, d.group_flags, d.hists, d.hist_items, mpf);
   if (marks) cudaEventRecord(marks[1], s);
-  batch_plan_encode_kernel<<<grid_of(c, kStagePlanEnc, count), 256, 0, s>>>(
-      d.items, d.states, count, d.ctrl, d.item_flags, d.hists, d.hist_items);
+  go(batch_plan_encode_kernel, grid_of(c, kStagePlanEnc, count), 256, 0, d.items, d.states, count,
+     d.ctrl, d.item_flags, d.hists, d.hist_items);
   if (marks) cudaEventRecord(marks[2], s);
-  batch_encode_kernel<<<grid_of(c, kStageEncode, div_up_u64(max_blocks, kBWarps)), kBThreads,
-                        sizeof(BatchEncSmem), s>>>(d.items, d.states, count, d.ctrl,
-                                                   d.block_flags, d.slots,
-                                                   (uint32_t)c.prefetch[kStageEncode]);
+  go(batch_encode_kernel, grid_of(c, kStageEncode, div_up_u64(max_blocks, kBWarps)), kBThreads,
+     sizeof(BatchEncSmem), d.items, d.states, count, d.ctrl, d.block_flags, d.slots,
+     (uint32_t)c.prefetch[kStageEncode]);
   if (marks) cudaEventRecord(marks[3], s);
-  return cudaGetLastError();
+  return e;
 }
 
 cudaError_t launch_batch_decompress(const BatchDev& d, uint32_t count, const uint64_t groups[3],
@@ -910,13 +920,17 @@ cudaError_t launch_batch_decompress(const BatchDev& d, uint32_t count, const uin
   if (likely_blocks >= (uint64_t)c.sms * 2 * 64) chunk = 64;
   if (likely_blocks >= (uint64_t)c.sms * 4 * 128) chunk = 128;
   const uint64_t max_chunks = div_up_u64(max_blocks, chunk) + count;
+  cudaError_t e = cudaSuccess;
+  auto go = [&](auto* kernel, unsigned grid, unsigned block, size_t smem, auto... args) {
+    if (e == cudaSuccess) e = launch(kernel, grid, block, smem, s, args...);
+  };
   if (marks) cudaEventRecord(marks[0], s);
-  batch_begin_kernel<<<(count + 255) / 256 + 1, 256, 0, s>>>(d.states, count, d.ctrl);
-  batch_plan_decode_kernel<<<grid_of(c, kStagePlanDec, count), 32, 0, s>>>(
-      d.items, d.states, count, d.ctrl, d.item_flags, chunk);
+  go(batch_begin_kernel, (count + 255) / 256 + 1, 256, 0, d.states, count, d.ctrl);
+  go(batch_plan_decode_kernel, grid_of(c, kStagePlanDec, count), 32, 0, d.items, d.states, count,
+     d.ctrl, d.item_flags, chunk);
   if (marks) cudaEventRecord(marks[1], s);
-  batch_decode_kernel<<<grid_of(c, kStageDecode, max_chunks), kDThreads, sizeof(BatchDecSmem),
-                        s>>>(d.items, d.states, count, d.ctrl, chunk);
+  go(batch_decode_kernel, grid_of(c, kStageDecode, max_chunks), kDThreads, sizeof(BatchDecSmem),
+     d.items, d.states, count, d.ctrl, chunk);
   if (marks) cudaEventRecord(marks[2], s);
   // runs of up to 16 units, while there are 8 for every warp of a full grid
   auto run_of = [&](uint64_t units) {
@@ -926,18 +940,18 @@ cudaError_t launch_batch_decompress(const BatchDev& d, uint32_t count, const uin
   };
   if (groups[1]) {
     const uint32_t r = run_of(groups[1]);
-    batch_unmap_kernel<MANS_U16><<<grid_of(c, kStageUnmap, div_up_u64(groups[1], (uint64_t)kBWarps * r),
-                                           c.occ_u16_unmap),
-                                   kBThreads, 0, s>>>(d.items, d.states, count, groups[1], d.ctrl, r);
+    go(batch_unmap_kernel<MANS_U16>,
+       grid_of(c, kStageUnmap, div_up_u64(groups[1], (uint64_t)kBWarps * r), c.occ_u16_unmap),
+       kBThreads, 0, d.items, d.states, count, groups[1], d.ctrl, r);
   }
   if (groups[2]) {
     const uint32_t r = run_of(groups[2]);
-    batch_unmap_kernel<MANS_U32><<<grid_of(c, kStageUnmap, div_up_u64(groups[2], (uint64_t)kBWarps * r)),
-                                   kBThreads, sizeof(BatchUnmapSmem), s>>>(d.items, d.states, count,
-                                                                          groups[2], d.ctrl, r);
+    go(batch_unmap_kernel<MANS_U32>,
+       grid_of(c, kStageUnmap, div_up_u64(groups[2], (uint64_t)kBWarps * r)), kBThreads,
+       sizeof(BatchUnmapSmem), d.items, d.states, count, groups[2], d.ctrl, r);
   }
   if (marks) cudaEventRecord(marks[3], s);
-  return cudaGetLastError();
+  return e;
 }
 
 }  // namespace mans
