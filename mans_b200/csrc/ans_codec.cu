@@ -265,10 +265,11 @@ __device__ __forceinline__ void decode_blocks(const uint8_t* __restrict__ in, ui
         if ((uint64_t)bn.y + wn <= cw) prefetch_l2(in + ans_overhead(nb) + 2ull * bn.y, 2 * wn);
       }
     };
-    if (kBlocks == 2 && take == 2 && b + 2 < nb) {
-      decode_block<kP, kBlocks>(in, nb, n, cw, out, lut, ws, b, lane, hook, bad);
-    } else {
-      // one by one; the last block may be short (and has no fixed chunks)
+    bool pair = kBlocks == 2 && take == 2 && b + 2 < nb;
+    if (pair) pair = decode_block<kP, kBlocks>(in, nb, n, cw, out, lut, ws, b, lane, hook, bad);
+    if (!pair) {
+      // one by one (the last block may be short, and has no fixed chunks); the
+      // hook has not run, so the next claim is made here
       for (uint32_t k = b; k < nb && k < b + take; ++k)
         decode_block<kP, 1>(in, nb, n, cw, out, lut, ws, k, lane, [](int) {}, bad);
       nxt = claim(b, nxt_take);

@@ -742,7 +742,10 @@ __device__ __forceinline__ uint32_t dec_lookup(uint32_t& x, const uint8_t* lut_l
 // into out + 4096 b. in: the stream (header validated by the caller: nb
 // blocks, n bytes, cw words); lut: its slot table for precision kP. A step is a chain of two shared-memory loads, a vote and
 // a population count; two blocks at a time give the warp two chains. With
-// kBlocks = 2 both blocks are full.
+// kBlocks = 2 both blocks are full, and where an entry of the two does not fit
+// the stream nothing is decoded or reported and the result is false: the
+// caller then takes the blocks one by one, so that a damaged block costs no
+// other. (kBlocks = 1: an entry that does not fit is reported.)
 // A corrupt stream can move the window's wa below the warp's words, by at most
 // 128 steps x 32 words = 8 KiB; the slot table (128 KiB) lies below
 // every warp's words in the CTA's shared memory, so such reads stay inside it,
@@ -751,7 +754,7 @@ __device__ __forceinline__ uint32_t dec_lookup(uint32_t& x, const uint8_t* lut_l
 // hook(c) runs before chunk c (the block's chunks count down to 0); bad(b) in
 // lane 0 reports block b as corrupt.
 template <int kP, int kBlocks, typename Stage, typename Hook, typename Bad>
-__device__ __forceinline__ void decode_block(const uint8_t* __restrict__ in, uint32_t nb, uint32_t n,
+__device__ __forceinline__ bool decode_block(const uint8_t* __restrict__ in, uint32_t nb, uint32_t n,
                                              uint32_t cw, uint8_t* __restrict__ out,
                                              const uint8_t* lut, Stage* ws, uint32_t b, int lane,
                                              Hook hook, Bad bad) {
@@ -760,10 +763,10 @@ __device__ __forceinline__ void decode_block(const uint8_t* __restrict__ in, uin
 #pragma unroll
   for (int u = 0; u < kBlocks; ++u) {
     const bool f = k[u].load(in, nb, n, cw, b + u, lane);
-    if (!f && lane == 0) bad(b + u);
+    if (kBlocks == 1 && !f && lane == 0) bad(b);
     fits = fits && f;
   }
-  if (!fits) return;
+  if (!fits) return false;
   uint8_t* dst = out + (uint64_t)b * kAnsBlock;
   const uint32_t gemask = lanemask_ge();
   const uint8_t* const ll = lut + 8u * (lane & ((1 << dec_copy_bits(kP)) - 1));
@@ -819,6 +822,7 @@ __device__ __forceinline__ void decode_block(const uint8_t* __restrict__ in, uin
     const bool ok = w[u].base == 0 && w[u].wa == w[u].wb && k[u].x == kAnsStartState;
     if (__any_sync(0xffffffffu, !ok) && lane == 0) bad(b + u);
   }
+  return true;
 }
 
 }  // namespace mans

@@ -604,9 +604,8 @@ __device__ __forceinline__ void batch_decode_chunk(const volatile BatchChunk& d,
                                                    Bad bad) {
   const uint32_t step = pairs ? 2u : 1u;
   for (uint32_t b = d.b0 + step * warp; b < d.b1; b += step * kDWarps) {
-    if (pairs && b + 2 < d.nb && b + 2 <= d.b1) {
-      decode_block<kP, 2>(d.in, d.nb, d.n, d.cw, d.out, lut, ws, b, lane, [](int) {}, bad);
-    } else {
+    if (!(pairs && b + 2 < d.nb && b + 2 <= d.b1 &&
+          decode_block<kP, 2>(d.in, d.nb, d.n, d.cw, d.out, lut, ws, b, lane, [](int) {}, bad))) {
 #pragma unroll 1
       for (uint32_t k = b; k < d.b1 && k < b + step; ++k)
         decode_block<kP, 1>(d.in, d.nb, d.n, d.cw, d.out, lut, ws, k, lane, [](int) {}, bad);
