@@ -298,9 +298,9 @@ mans_status mans_batch_stage_times(mans_batch* b, float ms[6], int calls[2]);
 mans_status mans_batch_get_schedule(const mans_batch* b, int ctas_per_sm[6],
                                     int max_ctas_per_sm[6]);
 mans_status mans_batch_set_schedule(mans_batch* b, const int ctas_per_sm[6]);
-/* The full schedule, per stage (same order): resident CTAs per SM (the map
- * stage counts CTAs of 8 warps), warps per CTA (4 or 8 for the map stage; the
- * others have a fixed number, given as 8) and the L2 prefetch distance in grids of units ahead (0 to
+/* The full schedule, per stage (same order): resident CTAs per SM (the map and
+ * decode stages count CTAs of 8 warps), warps per CTA (4 or 8 for the map stage,
+ * 8 for the others) and the L2 prefetch distance in grids of units ahead (0 to
  * 2 for the map and encode stages, 0 for the others). Never changes the bytes
  * produced. limits (may be NULL) receives the largest accepted values. */
 typedef struct mans_batch_schedule {

@@ -29,7 +29,9 @@ namespace mans {
 
 constexpr int kBWarps = 8;
 constexpr int kBThreads = kBWarps * 32;
-constexpr int kDWarps = 32;  // decode: one CTA per SM around one replicated table
+// decode: one CTA of up to 32 warps per SM around one replicated table (8 for
+// each CTA per SM of the schedule, which counts CTAs of 8 warps)
+constexpr int kDWarps = 32;
 constexpr int kDThreads = kDWarps * 32;
 constexpr uint32_t kRawChunk = 4096;  // histogram unit of a raw-byte buffer
 
@@ -603,7 +605,7 @@ __device__ __forceinline__ void batch_decode_chunk(const volatile BatchChunk& d,
                                                    DecWarp* ws, bool pairs, int warp, int lane,
                                                    Bad bad) {
   const uint32_t step = pairs ? 2u : 1u;
-  for (uint32_t b = d.b0 + step * warp; b < d.b1; b += step * kDWarps) {
+  for (uint32_t b = d.b0 + step * warp; b < d.b1; b += step * (blockDim.x >> 5)) {
     if (!(pairs && b + 2 < d.nb && b + 2 <= d.b1 &&
           decode_block<kP, 2>(d.in, d.nb, d.n, d.cw, d.out, lut, ws, b, lane, [](int) {}, bad))) {
 #pragma unroll 1
@@ -625,7 +627,8 @@ __global__ __launch_bounds__(kDThreads, 1) void batch_decode_kernel(const BatchI
   __shared__ uint32_t s_item, s_tables, s_cur;
   __shared__ int s_last;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const bool pairs = chunk_blocks > (uint32_t)kDWarps;
+  const uint32_t warps = blockDim.x >> 5;
+  const bool pairs = chunk_blocks > warps;
   auto base = [&](uint32_t i) { return (uint64_t)states[i].unit_base; };
   // Claim a chunk and describe it (thread 0).
   auto claim = [&](uint32_t slot) {
@@ -674,9 +677,9 @@ __global__ __launch_bounds__(kDThreads, 1) void batch_decode_kernel(const BatchI
     if (t == 0) claim(i == 0 ? 2 : i - 1);
     {
       const volatile BatchChunk& e = s_chunk[i == 2 ? 0 : i + 1];
-      // the warp's blocks of the next chunk: pairs at 2 (warp + 32 m), or one
-      const uint32_t k = e.b0 + (pairs ? 2u * warp + (lane & 1) + 64u * (lane >> 1)
-                                       : (uint32_t)(warp + 32 * lane));
+      // the warp's (first) blocks of the next chunk: pairs at 2 (warp + warps m), or one
+      const uint32_t k = e.b0 + (pairs ? 2u * (warp + warps * (lane >> 1)) + (lane & 1)
+                                       : warp + warps * lane);
       if (lane < 4 && k < e.b1) {
         const uint8_t* pst = e.in + kAnsHeaderBytes + 2 * kAnsSyms;
         const uint32_t nb = e.nb;
@@ -840,7 +843,8 @@ void init_batch_cfg(BatchCfg& c, const LaunchCfg& base) {
   c.occ[kStagePlanEnc] = occ((const void*)batch_plan_encode_kernel, 256, 0);
   c.occ[kStageEncode] = occ((const void*)batch_encode_kernel, kBThreads, sizeof(BatchEncSmem));
   c.occ[kStagePlanDec] = occ((const void*)batch_plan_decode_kernel, 32, 0);
-  c.occ[kStageDecode] = occ((const void*)batch_decode_kernel, kDThreads, sizeof(BatchDecSmem));
+  c.occ[kStageDecode] =
+      kDWarps / kBWarps * occ((const void*)batch_decode_kernel, kDThreads, sizeof(BatchDecSmem));
   c.occ[kStageUnmap] = min(occ((const void*)batch_unmap_kernel<MANS_U16>, kBThreads, 0),
                            occ((const void*)batch_unmap_kernel<MANS_U32>, kBThreads,
                                sizeof(BatchUnmapSmem)));
@@ -928,8 +932,9 @@ cudaError_t launch_batch_decompress(const BatchDev& d, uint32_t count, const uin
   go(batch_plan_decode_kernel, grid_of(c, kStagePlanDec, count), 32, 0, d.items, d.states, count,
      d.ctrl, d.item_flags, chunk);
   if (marks) cudaEventRecord(marks[1], s);
-  go(batch_decode_kernel, grid_of(c, kStageDecode, max_chunks), kDThreads, sizeof(BatchDecSmem),
-     d.items, d.states, count, d.ctrl, chunk);
+  go(batch_decode_kernel, (unsigned)min_u64(max_chunks < 1 ? 1 : max_chunks, (uint64_t)c.sms),
+     (unsigned)c.ctas_per_sm[kStageDecode] * kBThreads, sizeof(BatchDecSmem), d.items, d.states,
+     count, d.ctrl, chunk);
   if (marks) cudaEventRecord(marks[2], s);
   // runs of up to 16 units, while there are 8 for every warp of a full grid
   auto run_of = [&](uint64_t units) {

@@ -68,10 +68,10 @@ enum BatchStage {
 };
 
 // Schedule of the batched kernels. The bytes produced do not depend on it.
-//   ctas_per_sm: resident CTAs per SM of each stage (<= occ); for the map
-//     stage counted in CTAs of 8 warps, whatever its warps per CTA.
-//   warps: warps per CTA (the map stage takes 4 or 8; the others have a fixed
-//     number, shown as 8).
+//   ctas_per_sm: resident CTAs per SM of each stage (<= occ); for the map and
+//     decode stages counted in CTAs of 8 warps, whatever their warps per CTA
+//     (the decode stage runs them as one CTA).
+//   warps: warps per CTA (the map stage takes 4 or 8; the others 8).
 //   prefetch: L2 prefetch distance of the map and encode stages, in grids of
 //     units ahead (0: none; at most kMaxPrefetch).
 struct BatchCfg {

@@ -298,3 +298,24 @@ def test_batch_full_schedule_keeps_bytes(ws, torch_cuda):
                 b.set_schedule_ex(sch)
     finally:
         b.close()
+
+
+@pytest.mark.parametrize("decode", [1, 2, 3, 4])
+def test_batch_decode_stage_takes_one_to_four_ctas(ws, torch_cuda, decode):
+    """The decode stage counts resident CTAs of 8 warps, up to four: a schedule
+    kept from any of these is accepted and decodes to the same values."""
+    b = Batch(64, 64 << 20)
+    try:
+        xs = mixed(13, list(W.mixed_sizes(30, seed=13, lo=4 << 10, hi=2 << 20) // 4) + EDGE)
+        streams = [single_stream(ws, x, 10) for x in xs]
+        assert b.schedule()[1][4] == 4
+        b.set_schedule([3, 8, 4, 32, decode, 3])
+        assert b.schedule()[0][4] == decode
+        first, st, back = run_decompress(b, streams, xs)
+        assert first == 0, st
+        for x, y in zip(xs, back):
+            np.testing.assert_array_equal(y, x)
+        with pytest.raises(mb.MansError):
+            b.set_schedule([3, 8, 4, 32, 5, 3])
+    finally:
+        b.close()
