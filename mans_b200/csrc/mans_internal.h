@@ -35,7 +35,9 @@ inline cudaError_t launch(void (*kernel)(P...), unsigned grid, unsigned block, s
   cfg.stream = s;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();  // returned, not left for the caller's next check
+  return e;
 }
 
 struct LaunchCfg {
