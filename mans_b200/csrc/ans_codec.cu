@@ -14,6 +14,7 @@
 //    of device asserts, and checks that every block consumes exactly its
 //    words and returns to the start state.
 #include "ans_dev.cuh"
+#include <cstdlib>
 #include "mans_internal.h"
 
 namespace mans {
@@ -201,43 +202,48 @@ __global__ __launch_bounds__(kEncThreads) void ans_encode_shared_kernel(
 
 // ------------------------------------------------------------------------
 // Decode: a warp decodes a block, or two together, from the last step to the
-// first. One CTA of up to 32 warps per SM shares the replicated slot table
-// (128 KiB). What bounds it: per step 22 instructions (block overhead included)
-// of which 7 go to the half-rate integer ALU, two population counts, and a chain of two
-// shared-memory loads, a vote and a population count (about 130 cycles) that
-// only other chains can hide. The former kernel (22 instructions, 12 of them
-// ALU, table conflicts on 40% of its shared wavefronts, 32 chains per SM
-// instead of 64) took 0.575 ms on 1 GiB of detector frames (here 0.525), 1.092
-// on a 2 GiB uint16 volume (1.042), 27.7 us on 8 MiB of uint16 (21.0) and 131 us
-// on 100 MB of skewed bytes at p = 11 (105; its drop-in call also launched half
-// a resident wave). A single block takes 14.4 us instead of 13.4.
+// first. What bounds it: per step 22 instructions (block overhead included) of
+// which 7 go to the half-rate integer ALU, two population counts, the lookup's
+// shared-memory wavefronts, and a chain of two shared-memory loads, a vote and a
+// population count (about 130 cycles) that only other chains can hide. Two
+// kernels:
+//  * full: one CTA of 32 warps per SM around a replicated table of 128 KiB,
+//    pairs of blocks;
+//  * light: CTAs of eight warps, three to an SM, one copy of the 4-byte table,
+//    each block's words staged whole, a block per warp. Its table is built sooner,
+//    and kernels of several streams share an SM, for which the full one leaves
+//    no room.
 // ------------------------------------------------------------------------
-constexpr int kDecMaxWarps = 32, kDecMinWarps = 8;
-constexpr size_t kDecStageMax = (size_t)kDecMaxWarps * 2 * sizeof(DecWarp);
-constexpr size_t dec_stage_bytes(size_t warps, int blocks) {
-  return warps * sizeof(DecWhole) <= kDecStageMax ? warps * sizeof(DecWhole)
-                                                  : warps * blocks * sizeof(DecWarp);
-}
+constexpr int kDecFullWarps = 32, kDecLightWarps = 8, kDecLightCtas = 3;
+constexpr size_t kDecFullStage = (size_t)kDecFullWarps * 2 * sizeof(DecWarp);
+constexpr size_t kDecLightStage = (size_t)kDecLightWarps * sizeof(DecWhole);
+constexpr size_t kDecFullSmem = kDecLutBytes + kDecFullStage;
+constexpr size_t kDecLightSmem = kDecLutOneBytes + kDecLightStage;
 
-// kBlocks: blocks that a warp takes at a time and decodes together (one at a
-// time once less than a block per warp of the grid is left, so that the last
-// wave is short). Each warp's first blocks are fixed, spread over the CTAs, and
-// the rest is claimed: a small input then takes no claim at all (4,736 warps on
-// one counter cost 5 us). The next claim and its prefetches come in the middle
-// of the current blocks, where other warps hide their latency.
-template <int kP, int kBlocks>
+// Each warp's first blocks are fixed and the rest is claimed: a small input then
+// takes no claim at all (4,736 warps on one counter cost 5 us). They are spread
+// over the CTAs, or (`spread` false) fill CTA by CTA, so that a small input builds
+// few tables (four streams of 8 MiB uint16 calls: 11.4 us a call, spread 16.8).
+// Full: two blocks are taken at a time and decoded together,
+// one at a time once less than a block per warp of the grid is left, so that the
+// last wave is short. The next claim and its prefetches come in the middle of
+// the current blocks, where other warps hide their latency.
+template <int kP, bool kLight>
 __device__ __forceinline__ void decode_blocks(const uint8_t* __restrict__ in, uint32_t nb, uint32_t n,
                                               uint32_t cw, uint8_t* __restrict__ out,
-                                              const uint8_t* lut, uint8_t* stage, uint32_t stage_bytes,
+                                              const uint8_t* lut, uint8_t* stage, bool spread,
                                               Ctrl* ctrl, const Sink& sink, int lane) {
+  constexpr int kBlocks = kLight ? 1 : 2;
+  constexpr DecTab kTab = kLight ? kTabOne : dec_many(kP);
+  constexpr uint32_t kWhole = (kLight ? kDecLightStage : kDecFullStage) / sizeof(DecWhole);
   auto bad = [&](uint32_t k) { report(sink, MANS_ERR_CORRUPT, k); };
   const uint32_t warp = threadIdx.x >> 5;
-  if ((uint64_t)stage_bytes / sizeof(DecWhole) * gridDim.x >= nb) {
+  const uint32_t order = spread ? warp * gridDim.x + blockIdx.x : blockIdx.x * kDecLightWarps + warp;
+  if ((uint64_t)kWhole * gridDim.x >= nb) {
     // a block per warp at most, and room to stage its words whole
-    const uint32_t k = warp * gridDim.x + blockIdx.x;
-    if (k < nb)
-      decode_block<kP, 1>(in, nb, n, cw, out, lut, reinterpret_cast<DecWhole*>(stage) + warp, k, lane,
-                          [](int) {}, bad);
+    if (order < nb)
+      decode_block<kP, kTab, 1>(in, nb, n, cw, out, lut, reinterpret_cast<DecWhole*>(stage) + warp,
+                                order, lane, [](int) {}, bad);
     return;
   }
   DecWarp* const ws = reinterpret_cast<DecWarp*>(stage) + kBlocks * warp;
@@ -252,9 +258,9 @@ __device__ __forceinline__ void decode_blocks(const uint8_t* __restrict__ in, ui
     return __shfl_sync(0xffffffffu, v, 0);
   };
   uint32_t take = first;
-  uint32_t b = first * (warp * gridDim.x + blockIdx.x);
+  uint32_t b = first * order;
   while (b < nb) {
-    uint32_t nxt = 0, nxt_take = 0;
+    uint32_t nxt = 0, nxt_take = 0;  // nxt_take 0: not claimed yet
     auto hook = [&](int c) {
       if (c != 3) return;
       nxt = claim(b, nxt_take);
@@ -265,31 +271,33 @@ __device__ __forceinline__ void decode_blocks(const uint8_t* __restrict__ in, ui
         if ((uint64_t)bn.y + wn <= cw) prefetch_l2(in + ans_overhead(nb) + 2ull * bn.y, 2 * wn);
       }
     };
-    bool pair = kBlocks == 2 && take == 2 && b + 2 < nb;
-    if (pair) pair = decode_block<kP, kBlocks>(in, nb, n, cw, out, lut, ws, b, lane, hook, bad);
-    if (!pair) {
-      // one by one (the last block may be short, and has no fixed chunks); the
-      // hook has not run, so the next claim is made here
-      for (uint32_t k = b; k < nb && k < b + take; ++k)
-        decode_block<kP, 1>(in, nb, n, cw, out, lut, ws, k, lane, [](int) {}, bad);
-      nxt = claim(b, nxt_take);
+    if constexpr (kLight) {
+      decode_block<kP, kTab, 1>(in, nb, n, cw, out, lut, ws, b, lane, hook, bad);
+    } else {
+      bool pair = take == 2 && b + 2 < nb;
+      if (pair) pair = decode_block<kP, kTab, 2>(in, nb, n, cw, out, lut, ws, b, lane, hook, bad);
+      if (!pair)  // one by one (the last block may be short, and has no fixed chunks)
+        for (uint32_t k = b; k < nb && k < b + take; ++k)
+          decode_block<kP, kTab, 1>(in, nb, n, cw, out, lut, ws, k, lane, [](int) {}, bad);
     }
+    if (!nxt_take) nxt = claim(b, nxt_take);  // the hook has not run
     b = nxt;
     take = nxt_take;
   }
 }
 
-template <int kBlocks>
-__global__ __launch_bounds__(kDecMaxWarps * 32, 1) void ans_decode_kernel(
+template <bool kLight>
+__global__ __launch_bounds__((kLight ? kDecLightWarps : kDecFullWarps) * 32,
+                             kLight ? kDecLightCtas : 1) void ans_decode_kernel(
     const uint8_t* __restrict__ in, uint64_t in_size, uint8_t* __restrict__ out, uint64_t out_cap,
-    Ctrl* ctrl, int expect_p, int record, uint32_t stage_bytes) {
+    Ctrl* ctrl, int expect_p, int record) {
   kernel_begin();
   extern __shared__ __align__(16) uint8_t smem_raw[];
   __shared__ uint32_t s_incl[kAnsSyms];
   __shared__ int s_ok;
   const int t = threadIdx.x, lane = t & 31;
   uint8_t* const lut = smem_raw;  // below every warp's words (see decode_block)
-  uint8_t* const stage = smem_raw + kDecLutBytes;
+  uint8_t* const stage = smem_raw + (kLight ? kDecLutOneBytes : kDecLutBytes);
   const Sink sink = sink_of(ctrl);
 
   // ---- header validation (GpuANSCodec.h:106-113 asserts, GpuANSDecode.h:220-227)
@@ -312,15 +320,20 @@ __global__ __launch_bounds__(kDecMaxWarps * 32, 1) void ans_decode_kernel(
   if (record && ok && blockIdx.x == 0 && t == 0) ctrl->merged_size = n;
   __syncthreads();
 
-  if (s_ok && blockIdx.x < nb) {  // CTA k holds block k at least
-    const bool tables_ok = dec_build_lut(pdf, p, lut, s_incl);
+  // A CTA without a block builds no table. The light kernel fills CTA by CTA up to
+  // two thirds of the grid's warps (two CTAs per SM) and spreads the blocks from
+  // there on, so that the SMs have the same number (10 MB of bytes: 17.0 us a call,
+  // filled 17.5).
+  const bool spread = !kLight || 3ull * nb > 2ull * kDecLightWarps * gridDim.x;
+  if (s_ok && (spread ? blockIdx.x : blockIdx.x * kDecLightWarps) < nb) {
+    const bool tables_ok = dec_build_lut(pdf, p, kLight ? kTabOne : dec_many(p), lut, s_incl);
     if (!tables_ok && blockIdx.x == 0 && t == 0) report(sink, MANS_ERR_BAD_STREAM, 1);
     __syncthreads();
     if (tables_ok) {
       switch (p) {
-        case 9: decode_blocks<9, kBlocks>(in, nb, n, cw, out, lut, stage, stage_bytes, ctrl, sink, lane); break;
-        case 10: decode_blocks<10, kBlocks>(in, nb, n, cw, out, lut, stage, stage_bytes, ctrl, sink, lane); break;
-        default: decode_blocks<11, kBlocks>(in, nb, n, cw, out, lut, stage, stage_bytes, ctrl, sink, lane); break;
+        case 9: decode_blocks<9, kLight>(in, nb, n, cw, out, lut, stage, spread, ctrl, sink, lane); break;
+        case 10: decode_blocks<10, kLight>(in, nb, n, cw, out, lut, stage, spread, ctrl, sink, lane); break;
+        default: decode_blocks<11, kLight>(in, nb, n, cw, out, lut, stage, spread, ctrl, sink, lane); break;
       }
     }
   }
@@ -353,10 +366,10 @@ void init_ans_launch_cfg(LaunchCfg& cfg) {
   cudaFuncSetAttribute(ans_encode_shared_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(EncSmem));
   cfg.enc_ctas = occupancy((const void*)ans_encode_shared_kernel, kEncThreads, sizeof(EncSmem));
-  cudaFuncSetAttribute(ans_decode_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(kDecLutBytes + kDecStageMax));
-  cudaFuncSetAttribute(ans_decode_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(kDecLutBytes + kDecStageMax));
+  cudaFuncSetAttribute(ans_decode_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)kDecLightSmem);
+  cudaFuncSetAttribute(ans_decode_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)kDecFullSmem);
   cfg.hist_ctas = occupancy((const void*)hist_bytes_kernel, kHistThreads, 0);
 }
 
@@ -402,23 +415,28 @@ cudaError_t launch_ans_encode(const uint8_t* in, uint8_t* out, uint64_t out_cap,
   }
 }
 
+// Up to this many likely blocks per SM (its resident warps) the light kernel
+// decodes them. Per call, light / full: 4 MiB of bytes 14.6 / 15.5 us, 8 MB 15.4 /
+// 15.6, 12 MB 17.9 / 18.1; four streams of 16 MiB uint32 calls 24.4 / 28.5, of 12 MB
+// of bytes 15.4 / 17.0. With more blocks its warps take several (32 MiB of uint32
+// frames, 37 per SM: 47.7 / 43.3).
+constexpr uint64_t kDecLightBlocks = (uint64_t)kDecLightWarps * kDecLightCtas;
+
 cudaError_t launch_ans_decode(const uint8_t* in, uint64_t in_size, uint8_t* out, uint64_t out_cap,
                               Ctrl* ctrl, int expect_p, int record, uint64_t likely_blocks,
                               uint64_t max_blocks, const LaunchCfg& cfg, cudaStream_t s) {
-  // One CTA per SM with as many warps as spread the blocks evenly; a warp takes
-  // two blocks together once a block per warp does not hold them all (16 M
-  // uint16 values, 30 blocks per SM: decode 31 us one by one, 36 in pairs; 24 M,
-  // 45 per SM: 50 and 40; 1 GiB of detector frames: 0.591 and 0.525 ms).
-  const int blocks = likely_blocks > (uint64_t)cfg.sms * kDecMaxWarps ? 2 : 1;
-  uint64_t warps = div_up_u64(likely_blocks, (uint64_t)cfg.sms * blocks);
-  warps = warps < kDecMinWarps ? kDecMinWarps : warps < kDecMaxWarps ? warps : kDecMaxWarps;
-  const uint64_t want = div_up_u64(max_blocks, warps * blocks);
-  const unsigned grid =
-      (unsigned)(want < 1 ? 1 : (want < (uint64_t)cfg.sms ? want : (uint64_t)cfg.sms));
-  auto* k = blocks == 2 ? ans_decode_kernel<2> : ans_decode_kernel<1>;
-  const size_t stage = dec_stage_bytes(warps, blocks);
-  return launch(k, grid, (unsigned)warps * 32, kDecLutBytes + stage, s, in, in_size, out, out_cap,
-                ctrl, expect_p, record, (uint32_t)stage);
+  const uint64_t sms = (uint64_t)cfg.sms;
+  const bool light = likely_blocks <= sms * kDecLightBlocks;
+  // more than two CTAs per SM: as many as fit, so that every SM has the same number
+  const bool even = light && likely_blocks > sms * kDecLightWarps * (kDecLightCtas - 1);
+  const uint64_t want = light && !even ? div_up_u64(max_blocks, kDecLightWarps) : max_blocks;
+  const uint64_t cap = light ? sms * kDecLightCtas : sms;
+  const unsigned grid = (unsigned)(want < 1 ? 1 : (want < cap ? want : cap));
+  if (light)
+    return launch(ans_decode_kernel<true>, grid, kDecLightWarps * 32, kDecLightSmem, s, in, in_size,
+                  out, out_cap, ctrl, expect_p, record);
+  return launch(ans_decode_kernel<false>, grid, kDecFullWarps * 32, kDecFullSmem, s, in, in_size, out,
+                out_cap, ctrl, expect_p, record);
 }
 
 }  // namespace mans

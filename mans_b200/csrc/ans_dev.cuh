@@ -511,20 +511,27 @@ __device__ __forceinline__ void encode_block(
 // ---- decode ----
 constexpr int kMaxProbBits = 11;
 
-// The slot table of a stream's pdf, 8 bytes per slot s of symbol y:
-//   {P = pdf << (32 - p), D << 8 | y}, D = (s - cdf) - (s * pdf >> p) (signed),
-// so that the decoder's new state pdf * (x >> p) + (s - cdf), s = x mod 2^p
-// (GpuANSDecode.h:307-377), is umulhi(x, P) + D: umulhi(x, P) = x * pdf >> p =
-// pdf * (x >> p) + (s * pdf >> p), exactly, and the second term depends on s
-// alone. (pdf = 2^p, a single symbol: P = 2^32 - 1 and D = 1, since the state
-// x >= 1 stays as it is.)
-// The table is kept in 16 copies (p <= 10) or 8 (p = 11): with n copies, copy c
-// of slot s at byte 8 (n s + c). Slots are uniformly distributed whatever the data, so
-// with one copy the 32 lookups of a step take about 6 shared-memory
-// wavefronts; a lane that reads its own copy (lane modulo the copies) takes 2
-// (16 copies) or 4 (8).
-constexpr uint32_t kDecLutBytes = 128u << 10;
-__host__ __device__ constexpr int dec_copy_bits(int p) { return p <= 10 ? 4 : 3; }
+// The slot table of a stream's pdf: for slot s = x mod 2^p of symbol y, what
+// turns the state x into pdf * (x >> p) + (s - cdf) (GpuANSDecode.h:307-377).
+// Slots are uniformly distributed whatever the data, so with one copy the 32
+// lookups of a step conflict; a lane that reads its own copy (lane modulo the
+// copies) takes fewer shared-memory wavefronts. Three forms:
+//  kTabWide: {P = pdf << (32 - p), D << 8 | y}, D = (s - cdf) - (s * pdf >> p)
+//    (signed): the new state is umulhi(x, P) + D, since umulhi(x, P) = x * pdf
+//    >> p = pdf * (x >> p) + (s * pdf >> p), exactly, and the second term depends
+//    on s alone. (pdf = 2^p, a single symbol: P = 2^32 - 1 and D = 1, since the
+//    state x >= 1 stays as it is.) 8 bytes, 16 copies, 2 wavefronts: the fewest
+//    instructions, for p <= 10.
+//  kTabMany: {s - cdf:12, y:8, pdf:12} (one instruction per field, and one between
+//    the load and the multiplication), 4 bytes, 16 copies, 2 wavefronts: for p =
+//    11, where the wide form has room for 8 copies only (4 wavefronts).
+//  kTabOne: the same entries, one copy (about 3.5 wavefronts): at most 8 KiB, quick
+//    to build and small beside other kernels on the SM.
+enum DecTab { kTabWide, kTabMany, kTabOne };
+constexpr int kDecCopyBits = 4;
+constexpr uint32_t kDecLutBytes = 128u << 10;                // kTabWide, kTabMany
+constexpr uint32_t kDecLutOneBytes = 4u << kMaxProbBits;     // kTabOne
+__host__ __device__ constexpr DecTab dec_many(int p) { return p <= 10 ? kTabWide : kTabMany; }
 __device__ __forceinline__ uint2 make_dec_entry(uint32_t pdf, uint32_t s, uint32_t cdf, uint32_t sym,
                                                 int p) {
   if (pdf >> p) return make_uint2(0xffffffffu, (1u << 8) | sym);
@@ -541,7 +548,7 @@ __device__ __forceinline__ uint32_t dec_pdf(const uint8_t* __restrict__ in) {
              ? __ldg(reinterpret_cast<const uint16_t*>(in + kAnsHeaderBytes) + threadIdx.x)
              : 0u;
 }
-__device__ __forceinline__ bool dec_build_lut(uint32_t pdf, int p, uint8_t* lut,
+__device__ __forceinline__ bool dec_build_lut(uint32_t pdf, int p, DecTab tab, uint8_t* lut,
                                               uint32_t* s_incl) {
   __shared__ uint32_t s_sum[8];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -572,11 +579,16 @@ __device__ __forceinline__ bool dec_build_lut(uint32_t pdf, int p, uint8_t* lut,
     for (uint32_t h = 128; h > 0; h >>= 1)
       if (s_incl[sym + h - 1] <= s) sym += h;
     const uint32_t hi = s_incl[sym], lo = sym ? s_incl[sym - 1] : 0u;
-    const uint2 e = make_dec_entry(hi - lo, s, lo, sym, p);
-    // a row of copies, rotated so that the lanes of a store spread over the banks
-    const uint32_t n16 = 1u << (dec_copy_bits(p) - 1);
-    uint4* row = reinterpret_cast<uint4*>(lut) + s * n16;
-    for (uint32_t c = 0; c < n16; ++c) row[(c + lane) & (n16 - 1)] = make_uint4(e.x, e.y, e.x, e.y);
+    const uint32_t e = (s - lo) << 20 | sym << 12 | (hi - lo);
+    if (tab == kTabOne) {
+      reinterpret_cast<uint32_t*>(lut)[s] = e;
+    } else {
+      // a row of copies, rotated so that the lanes of a store spread over the banks
+      const uint2 w = tab == kTabWide ? make_dec_entry(hi - lo, s, lo, sym, p) : make_uint2(e, e);
+      const uint32_t n16 = tab == kTabWide ? 8u : 4u;
+      uint4* row = reinterpret_cast<uint4*>(lut) + s * n16;
+      for (uint32_t c = 0; c < n16; ++c) row[(c + lane) & (n16 - 1)] = make_uint4(w.x, w.y, w.x, w.y);
+    }
   }
   return true;
 }
@@ -729,13 +741,22 @@ struct DecBlock {
   }
 };
 
-// One step's lookup: slot of the state, table entry, new state.
-template <int kP>
+// One step's lookup: slot of the state, table entry, new state. Returns the
+// symbol in the low byte.
+template <int kP, DecTab kTab>
 __device__ __forceinline__ uint32_t dec_lookup(uint32_t& x, const uint8_t* lut_lane) {
-  constexpr uint32_t kShift = dec_copy_bits(kP) + 3, kMask = ((1u << kP) - 1u) << kShift;
-  const uint2 e = *reinterpret_cast<const uint2*>(lut_lane + ((x << kShift) & kMask));
-  asm("mad.hi.u32 %0, %0, %1, %2;" : "+r"(x) : "r"(e.x), "r"((uint32_t)((int)e.y >> 8)));
-  return e.y;
+  constexpr uint32_t kShift = (kTab == kTabWide ? 3 : 2) + (kTab == kTabOne ? 0 : kDecCopyBits);
+  constexpr uint32_t kMask = ((1u << kP) - 1u) << kShift;
+  const uint8_t* const at = lut_lane + ((x << kShift) & kMask);
+  if constexpr (kTab == kTabWide) {
+    const uint2 e = *reinterpret_cast<const uint2*>(at);
+    asm("mad.hi.u32 %0, %0, %1, %2;" : "+r"(x) : "r"(e.x), "r"((uint32_t)((int)e.y >> 8)));
+    return e.y;
+  } else {
+    const uint32_t e = *reinterpret_cast<const uint32_t*>(at);
+    x = (e & 0xfffu) * (x >> kP) + (e >> 20);
+    return e >> 12;
+  }
 }
 
 // Decode kBlocks (1 or 2) consecutive blocks, b on, of one stream (one warp)
@@ -747,13 +768,13 @@ __device__ __forceinline__ uint32_t dec_lookup(uint32_t& x, const uint8_t* lut_l
 // caller then takes the blocks one by one, so that a damaged block costs no
 // other. (kBlocks = 1: an entry that does not fit is reported.)
 // A corrupt stream can move the window's wa below the warp's words, by at most
-// 128 steps x 32 words = 8 KiB; the slot table (128 KiB) lies below
-// every warp's words in the CTA's shared memory, so such reads stay inside it,
-// and the final position check reports the block.
+// 128 steps x 32 words = 8 KiB; the slot table's memory (8 KiB at least) lies
+// below every warp's words in the CTA's shared memory, so such reads stay
+// inside it, and the final position check reports the block.
 // Stage: DecWarp (kBlocks of them) or DecWhole, the warp's shared memory.
 // hook(c) runs before chunk c (the block's chunks count down to 0); bad(b) in
 // lane 0 reports block b as corrupt.
-template <int kP, int kBlocks, typename Stage, typename Hook, typename Bad>
+template <int kP, DecTab kTab, int kBlocks, typename Stage, typename Hook, typename Bad>
 __device__ __forceinline__ bool decode_block(const uint8_t* __restrict__ in, uint32_t nb, uint32_t n,
                                              uint32_t cw, uint8_t* __restrict__ out,
                                              const uint8_t* lut, Stage* ws, uint32_t b, int lane,
@@ -769,7 +790,8 @@ __device__ __forceinline__ bool decode_block(const uint8_t* __restrict__ in, uin
   if (!fits) return false;
   uint8_t* dst = out + (uint64_t)b * kAnsBlock;
   const uint32_t gemask = lanemask_ge();
-  const uint8_t* const ll = lut + 8u * (lane & ((1 << dec_copy_bits(kP)) - 1));
+  const uint8_t* const ll = lut + (kTab == kTabWide ? 8u : 4u) *
+                                      (kTab == kTabOne ? 0u : lane & ((1u << kDecCopyBits) - 1));
   DecWindow w[kBlocks];
   __syncwarp();
 #pragma unroll
@@ -789,7 +811,7 @@ __device__ __forceinline__ bool decode_block(const uint8_t* __restrict__ in, uin
       const bool valid = 32u * j + lane < bs;
       if (valid) {
         xs = k[0].x;
-        dst[j * 32 + lane] = (uint8_t)dec_lookup<kP>(xs, ll);
+        dst[j * 32 + lane] = (uint8_t)dec_lookup<kP, kTab>(xs, ll);
       }
       dec_read(xs, w[0].wa, gemask);
       if (valid) k[0].x = xs;
@@ -807,7 +829,7 @@ __device__ __forceinline__ bool decode_block(const uint8_t* __restrict__ in, uin
       }
 #pragma unroll
       for (int u = 0; u < kBlocks; ++u)
-        ws[u].out[ph + lane + i * 32] = (uint8_t)dec_lookup<kP>(k[u].x, ll);
+        ws[u].out[ph + lane + i * 32] = (uint8_t)dec_lookup<kP, kTab>(k[u].x, ll);
 #pragma unroll
       for (int u = 0; u < kBlocks; ++u) dec_read(k[u].x, w[u].wa, gemask);
     }

@@ -607,10 +607,11 @@ __device__ __forceinline__ void batch_decode_chunk(const volatile BatchChunk& d,
   const uint32_t step = pairs ? 2u : 1u;
   for (uint32_t b = d.b0 + step * warp; b < d.b1; b += step * (blockDim.x >> 5)) {
     if (!(pairs && b + 2 < d.nb && b + 2 <= d.b1 &&
-          decode_block<kP, 2>(d.in, d.nb, d.n, d.cw, d.out, lut, ws, b, lane, [](int) {}, bad))) {
+          decode_block<kP, dec_many(kP), 2>(d.in, d.nb, d.n, d.cw, d.out, lut, ws, b, lane, [](int) {}, bad))) {
 #pragma unroll 1
       for (uint32_t k = b; k < d.b1 && k < b + step; ++k)
-        decode_block<kP, 1>(d.in, d.nb, d.n, d.cw, d.out, lut, ws, k, lane, [](int) {}, bad);
+        decode_block<kP, dec_many(kP), 1>(d.in, d.nb, d.n, d.cw, d.out, lut, ws, k, lane, [](int) {},
+                                          bad);
     }
   }
 }
@@ -666,7 +667,7 @@ __global__ __launch_bounds__(kDThreads, 1) void batch_decode_kernel(const BatchI
     const volatile BatchChunk& d = s_chunk[i];
     if (d.b0 == d.b1) break;
     if (s_cur != d.item) {
-      const bool ok = dec_build_lut(dec_pdf(d.in), (int)d.p, sm.lut, s_incl);
+      const bool ok = dec_build_lut(dec_pdf(d.in), (int)d.p, dec_many(d.p), sm.lut, s_incl);
       if (t == 0) s_tables = ok;
       __syncthreads();
       if (t == 0) {

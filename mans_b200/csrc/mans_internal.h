@@ -80,7 +80,8 @@ cudaError_t launch_ans_encode(const uint8_t* in, uint8_t* out, uint64_t out_cap,
 uint64_t ans_encode_slot_bytes(const LaunchCfg& cfg);
 // Decode the stream at `in` into `out` (at most out_cap bytes). expect_p < 0
 // accepts any valid precision. record != 0 stores the decoded size in ctrl.
-// likely_blocks and max_blocks: as in launch_ans_encode.
+// likely_blocks: what is to be expected (which of two kernels); max_blocks: as
+// in launch_ans_encode.
 cudaError_t launch_ans_decode(const uint8_t* in, uint64_t in_size, uint8_t* out, uint64_t out_cap,
                               Ctrl* ctrl, int expect_p, int record, uint64_t likely_blocks,
                               uint64_t max_blocks, const LaunchCfg& cfg, cudaStream_t s);

@@ -193,3 +193,50 @@ def test_u16_streams_around_their_word_limits(ws, oracle, b, layout):
     np.testing.assert_array_equal(to_host(s), oracle.compress(x, 10, layout))
     y = mb.decompress(s, n, torch.uint16, ws=ws, layout=layout)
     np.testing.assert_array_equal(to_host(y, np.uint16), x)
+
+
+@pytest.mark.parametrize("p", [9, 10, 11])
+@pytest.mark.parametrize("blocks", [1, 8, 9, 24 * SMS - 1, 24 * SMS, 24 * SMS + 1, 64 * SMS + 1])
+@pytest.mark.parametrize("tail", [0, -4090])
+def test_decoder_kernels(ws, oracle, blocks, tail, p):
+    """The decoder's two kernels (three CTAs of eight warps per multiprocessor,
+    or one of 32) at the sizes where one takes over from the other, full and
+    short last blocks."""
+    import torch
+    n = blocks * 4096 + tail
+    x = W.random_bytes(n, blocks + p, ("uniform", "sparse", "skewed")[p - 9])
+    s = to_dev(oracle.ans_encode(x, p))
+    for _ in range(2):  # the second call finds the work counters reset
+        np.testing.assert_array_equal(to_host(mb.decompress(s, n, torch.uint8, ws=ws)), x)
+
+
+@pytest.mark.parametrize("p", [9, 10, 11])
+@pytest.mark.parametrize("kind,n", [("wide", 3_400_000), ("wide", 4_700_001), ("near", 5_500_003)])
+def test_decoder_block_count_off_the_estimate(kind, n, p):
+    """Many more blocks than estimated from the value count (a warp of the small
+    kernel takes several), and many fewer (the large one's warps one at most).
+    The stream is the library's own; a damaged one is refused between."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    hi = 90 if kind == "near" else 2**31 - 1
+    x = torch.randint(0 if kind == "near" else -2**31, hi, (n,), dtype=torch.int32, device="cuda",
+                      generator=g).view(torch.uint32)
+    w = mb.Workspace(4 * n)
+    try:
+        s = mb.compress(x, p, ws=w)
+        nb = int(to_host(s[:32]).view(np.uint32)[1])
+        est = -(-3 * n // 4096)
+        if kind == "near":
+            assert nb < 15 * SMS and est > 24 * SMS
+        else:
+            assert nb > 24 * SMS and est <= 24 * SMS
+        bad = s.clone()
+        for b in (0, nb // 2, nb - 1):
+            bad[32 + 512 + 128 * nb + 8 * b + 2] ^= 1  # the block's byte count
+        y = torch.empty_like(x)
+        mb.decompress_into(w, bad, bad.numel(), y)
+        assert w.status()[0] == 10  # MANS_ERR_CORRUPT
+        assert torch.equal(mb.decompress(s, n, torch.uint32, ws=w), x)
+    finally:
+        w.close()
