@@ -67,7 +67,7 @@ __global__ __launch_bounds__(kHistThreads) void hist_bytes_kernel(const uint8_t*
 // ------------------------------------------------------------------------
 // One CTA of up to 32 warps per SM shares the 32 KiB table; small inputs take
 // smaller CTAs, so that their blocks spread over the SMs.
-constexpr int kEncMaxWarps = 32, kEncMaxThreads = kEncMaxWarps * 32;
+constexpr int kEncMinWarps = 4, kEncMaxWarps = 32, kEncMaxThreads = kEncMaxWarps * 32;
 
 // Empty input: header and a zero pdf only (GpuANSEncode.h:201-237).
 __device__ __forceinline__ void encode_empty(uint8_t* __restrict__ out, uint64_t out_cap, int p,
@@ -139,7 +139,11 @@ __global__ __launch_bounds__(kEncMaxThreads, 1) void ans_encode_slots_kernel(
       slots + ((uint64_t)blockIdx.x * warps + warp) * 2 * kEncSlotBytes);
   EncPending pend{0xffffffffu, 0, 0, nullptr};
   uint32_t cur = 0;
-  while (!failed) {
+  // Fewer blocks than warps were launched for: as many warps of every CTA as
+  // spread them evenly take part (claimed by all, the blocks crowd on the SMs
+  // that come first; 6 M small uint32 values 50.9 us a call, so 42.8).
+  const bool idle = failed || (warp >= kEncMinWarps && (uint64_t)warp * gridDim.x >= nb);
+  while (!idle) {
     const uint32_t b = warp_claim(&ctrl->tile_counter[1], lane);
     if (b >= nb) break;
     if (!kGather && lane == 0 && (uint64_t)b + ahead < nb) {
@@ -393,7 +397,7 @@ cudaError_t launch_ans_encode(const uint8_t* in, uint8_t* out, uint64_t out_cap,
   if (slots) {
     // one CTA per SM with as many warps as spread the blocks evenly
     uint64_t warps = div_up_u64(likely_blocks, (uint64_t)cfg.sms);
-    warps = warps < 4 ? 4 : warps < kEncMaxWarps ? warps : kEncMaxWarps;
+    warps = warps < kEncMinWarps ? kEncMinWarps : warps < kEncMaxWarps ? warps : kEncMaxWarps;
     const uint64_t want = div_up_u64(max_blocks, warps);
     const unsigned grid =
         (unsigned)(want < 1 ? 1 : (want < (uint64_t)cfg.sms ? want : (uint64_t)cfg.sms));

@@ -172,8 +172,8 @@ unsigned copy_grid(const LaunchCfg& cfg, uint64_t n) {
 // map, 51.7 so; 4 M: 75 and 69; 2^28: 1,587 and 1,340).
 constexpr uint64_t kSplitMin = 1u << 21;
 
-// 4 KiB blocks that n mapped elements are likely to have, for the shape of the
-// decoder's launch (more or fewer cost time only). Mapped bytes per element:
+// 4 KiB blocks that n mapped elements are likely to have, for the shapes of the
+// coder's launches (more or fewer cost time only). Mapped bytes per element:
 // uint16 volume 1.20, gradient 1.33, a spread of 2,000 3.34; uint32 detector
 // frames 2.68, Laplace codes 3.00, uniform values 5.08.
 uint64_t likely_blocks(mans_dtype dtype, uint64_t n) {
@@ -241,9 +241,8 @@ mans_status compress_impl(mans_workspace* ws, mans_dtype dtype, mans_layout layo
       e = launch(export_merged_kernel, copy_grid(ws->cfg, ws->merged_cap), 256, 0, s, m,
                  (uint8_t*)d_out, out_capacity, ws->ctrl, osz);
     } else {
-      // an element maps to one byte, and a little more
       e = launch_ans_encode(m, (uint8_t*)d_out, out_capacity, osz, nullptr, ws->ctrl,
-                            ws->ans_flags, precision, div_up_u64(n_elems + n_elems / 4, kAnsBlock),
+                            ws->ans_flags, precision, likely_blocks(dtype, n_elems),
                             div_up_u64(ws->merged_cap, kAnsBlock), ws->cfg, s, ws->enc_slots,
                             split ? &gather : nullptr);
     }

@@ -240,3 +240,23 @@ def test_decoder_block_count_off_the_estimate(kind, n, p):
         assert torch.equal(mb.decompress(s, n, torch.uint32, ws=w), x)
     finally:
         w.close()
+
+
+@pytest.mark.parametrize("kind", ["wide", "near", "quant"])
+@pytest.mark.parametrize("n", [150_000, 1_000_001, (1 << 21) - 1, 3 << 20])
+def test_encoder_block_count_off_the_estimate(oracle, n, kind):
+    """uint32 data of one to five mapped bytes a value, for which the encoder's
+    CTAs are launched alike: with blocks for some of their warps, all, or several
+    rounds, on both sides of the size from which it gathers the records."""
+    import torch
+    rng = np.random.default_rng(n)
+    x = {"wide": lambda: rng.integers(0, 1 << 32, n, dtype=np.uint64).astype(np.uint32),
+         "near": lambda: rng.integers(0, 90, n).astype(np.uint32),
+         "quant": lambda: W.quant_u32(n, 5)}[kind]()
+    w = mb.Workspace(4 * n)
+    try:
+        for p in (9, 11):
+            s = mb.compress(to_dev(x), p, ws=w)
+            np.testing.assert_array_equal(to_host(s), oracle.compress(x, p))
+    finally:
+        w.close()
