@@ -723,13 +723,15 @@ struct BatchUnmapSmem {
 
 // Runs of up to 16 units per claim, with the buffer's fields and checks loaded
 // when a warp comes to it instead of unit by unit (256 mixed buffers, 1.6 GB:
-// 1.296 -> 1.020 ms); uint16 at 4 CTAs per SM (64 registers; 3 CTAs: 1.146),
-// uint32 at 5.
+// 1.296 -> 1.020 ms); the last eighth of the units is claimed one by one, since a
+// unit of long lanes takes 150 us and a late run of them kept its warp alone
+// (1.015 -> 0.998 ms; 64 buffers of long lanes 9.71 -> 9.56, by units alone 9.49).
+// uint16 at 4 CTAs per SM (64 registers; 3 CTAs: 1.134), uint32 at 5.
 template <uint32_t kDtype>
 __global__ __launch_bounds__(kBThreads, kDtype == MANS_U16 ? 4 : 5) void batch_unmap_kernel(const BatchItem* __restrict__ items,
                                                                 BatchState* states, uint32_t count,
                                                                 uint64_t total_units, Ctrl* ctrl,
-                                                                uint32_t unit_run) {
+                                                                uint32_t unit_run, uint32_t runs) {
   kernel_begin();
   extern __shared__ __align__(16) uint8_t smem_raw[];
   __shared__ int s_last;
@@ -742,15 +744,18 @@ __global__ __launch_bounds__(kBThreads, kDtype == MANS_U16 ? 4 : 5) void batch_u
   uint64_t n = 0, size = 0, rest = 0, item_base = 0;  // size: bit bytes / 32, or record bytes
   bool skip = true;
   // Units do not depend on one another here (no look-back), so a warp claims
-  // unit_run consecutive ones at a time, and the next run while it restores
-  // the current one: the claim's round trip to L2 and the buffer's look-up
-  // leave the units' dependency chain.
+  // unit_run consecutive ones at a time (claims below `runs`; the others are for
+  // one unit), and the next run while it restores the current one: the claim's
+  // round trip to L2 and the buffer's look-up leave the units' dependency chain.
   uint32_t run = warp_claim(&ctrl->tile_counter[kSlot], lane);
-  while ((uint64_t)run * unit_run < total_units) {
+  while (true) {
+    const bool whole = run < runs;
+    const uint64_t u0 = whole ? (uint64_t)run * unit_run : (uint64_t)runs * unit_run + (run - runs);
+    if (u0 >= total_units) break;
     uint32_t nxt = 0;
     if (lane == 0) nxt = atomicAdd(&ctrl->tile_counter[kSlot], 1u);
-    const uint64_t u1 = min_u64(((uint64_t)run + 1) * unit_run, total_units);
-    for (uint64_t u = (uint64_t)run * unit_run; u < u1; ++u) {
+    const uint64_t u1 = u0 + (whole ? unit_run : 1u);
+    for (uint64_t u = u0; u < u1; ++u) {
       if (cur == 0xffffffffu || u >= rest) {  // past the current buffer's units
         for (uint32_t j = it + 1; j < count; ++j) {
           const BatchItem& x = items[j];
@@ -937,23 +942,27 @@ cudaError_t launch_batch_decompress(const BatchDev& d, uint32_t count, const uin
      (unsigned)c.ctas_per_sm[kStageDecode] * kBThreads, sizeof(BatchDecSmem), d.items, d.states,
      count, d.ctrl, chunk);
   if (marks) cudaEventRecord(marks[2], s);
-  // runs of up to 16 units, while there are 8 for every warp of a full grid
+  // runs of up to 16 units, while there are 8 for every warp of a full grid, for
+  // seven eighths of them
   auto run_of = [&](uint64_t units) {
     uint32_t r = 1;
     while (r < 16 && units >= (uint64_t)c.sms * 32 * 8 * 2 * r) r *= 2;
     return r;
   };
+  auto runs_of = [](uint64_t units, uint32_t r) {
+    return r == 1 ? 0u : (uint32_t)(units / r * 7 / 8);
+  };
   if (groups[1]) {
     const uint32_t r = run_of(groups[1]);
     go(batch_unmap_kernel<MANS_U16>,
        grid_of(c, kStageUnmap, div_up_u64(groups[1], (uint64_t)kBWarps * r), c.occ_u16_unmap),
-       kBThreads, 0, d.items, d.states, count, groups[1], d.ctrl, r);
+       kBThreads, 0, d.items, d.states, count, groups[1], d.ctrl, r, runs_of(groups[1], r));
   }
   if (groups[2]) {
     const uint32_t r = run_of(groups[2]);
     go(batch_unmap_kernel<MANS_U32>,
        grid_of(c, kStageUnmap, div_up_u64(groups[2], (uint64_t)kBWarps * r)), kBThreads,
-       sizeof(BatchUnmapSmem), d.items, d.states, count, groups[2], d.ctrl, r);
+       sizeof(BatchUnmapSmem), d.items, d.states, count, groups[2], d.ctrl, r, runs_of(groups[2], r));
   }
   if (marks) cudaEventRecord(marks[3], s);
   return e;

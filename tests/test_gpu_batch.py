@@ -319,3 +319,43 @@ def test_batch_decode_stage_takes_one_to_four_ctas(ws, torch_cuda, decode):
             b.set_schedule([3, 8, 4, 32, 5, 3])
     finally:
         b.close()
+
+
+@pytest.mark.parametrize("elem", [2, 4])
+@pytest.mark.parametrize("groups", [80_000, 160_000, 610_000])
+def test_batch_unmap_runs(torch_cuda, elem, groups):
+    """Enough groups of one type that the inverse mapping claims runs of 2, 4 and
+    16 of them: runs that cross into the next buffer, buffers smaller than a run,
+    empty ones, the single claims at the end, and a refused buffer between others."""
+    import torch
+    dt = torch.uint16 if elem == 2 else torch.uint32
+    small = [1, 511, 512, 0, 513, 512 * 15, 512 * 16, 512 * 16 + 1, 7, 512 * 33 + 5, 2]
+    ns = small * 3 + [groups // 2 * 512 - 77] + small * 9 + [groups // 2 * 512 + 300] + small * 2
+    g = torch.Generator(device="cuda")
+    g.manual_seed(groups + elem)
+    u = torch.rand(sum(ns), device="cuda", generator=g)
+    # most groups of one-byte codes, some values far away
+    v = (1000 + 90 * u + 7000 * (u > 0.9995)).to(torch.int32)
+    pool = v.to(torch.int16).view(dt) if elem == 2 else v.view(dt)
+    del u, v
+    xs = list(torch.split(pool, ns))
+    b = Batch(len(ns), pool.numel() * elem + 4096)
+    try:
+        streams = b.compress([x.clone() for x in xs])
+        bad = (34 + 11 * 4 + 5, 8)  # among the small ones between the large, and at the start
+        for i in bad:
+            streams[i] = streams[i].clone()
+            streams[i][3] ^= 0x40  # the magic
+        outs = [torch.full_like(x.view(torch.uint8), 77).view(dt) for x in xs]
+        for _ in range(2):
+            b.decompress_async(Batch.decompress_items(streams, [s.numel() for s in streams], outs))
+            _, st, _ = b.status(len(ns))
+            for i, (x, y) in enumerate(zip(xs, outs)):
+                if i in bad:
+                    assert mb.STATUS[st[i]] == "MANS_ERR_BAD_STREAM"
+                    assert bool((y.view(torch.uint8) == 77).all())
+                else:
+                    assert st[i] == 0
+                    assert torch.equal(y.view(torch.uint8), x.view(torch.uint8)), i
+    finally:
+        b.close()
