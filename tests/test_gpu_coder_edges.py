@@ -260,3 +260,43 @@ def test_encoder_block_count_off_the_estimate(oracle, n, kind):
             np.testing.assert_array_equal(to_host(s), oracle.compress(x, p))
     finally:
         w.close()
+
+
+def _groups_at_the_limits(n, seed):
+    """uint32 groups whose values reach exactly to 125, 126, 127 or 300 from their
+    center on either side, at low, middle and the highest centers; a few values of
+    every group sit at the limits, as many below as above, and the rest at the
+    center, so that the truncated mean is the center."""
+    rng = np.random.default_rng(seed)
+    x = np.empty(n, np.uint32)
+    for g in range(0, n, 512):
+        m = min(512, n - g)
+        d = int(rng.choice([0, 1, 125, 126, 127, 300]))
+        c = int(rng.choice([d, 130 + d, 70_000, 1 << 31, (1 << 32) - 1 - d]))
+        v = np.full(m, c, np.int64)
+        k = int(rng.integers(0, min(m // 2, 9)))
+        at = rng.permutation(m)
+        v[at[:k]] = c - d
+        v[at[k:2 * k]] = c + d
+        x[g:g + m] = v
+    return x
+
+
+@pytest.mark.parametrize("p", [9, 10, 11])
+@pytest.mark.parametrize("n", [(1 << 21) - 512, 1 << 21, (1 << 21) + 300])
+def test_u32_split_groups_at_the_limits(oracle, n, p):
+    """The short path of the uint32 map that leaves records in slots, at its
+    limits, and the gathering encoder at every precision."""
+    import torch
+    x = _groups_at_the_limits(n, n + p)
+    assert int(x.min()) == 0 and int(x.max()) == (1 << 32) - 1
+    codes = oracle.adm_u32_map(x[:1 << 20])
+    assert (codes == 253).any() and (codes == 252).any()  # 126 below and above
+    w = mb.Workspace(4 * n)
+    try:
+        s = mb.compress(to_dev(x), p, ws=w)
+        np.testing.assert_array_equal(to_host(s), oracle.compress(x, p))
+        y = mb.decompress(s, n, torch.uint32, ws=w)
+    finally:
+        w.close()
+    np.testing.assert_array_equal(to_host(y, np.uint32), x)
