@@ -351,6 +351,14 @@ def run_reference(args):
 
 
 # ---------------------------------------------------------------- GPU arm
+def splits_u32_map(n: int) -> bool:
+    """Whether a compress of n uint32 values on a default workspace maps with two
+    kernels (the second a scan): from 2 M values on, while the records' slots (4,136
+    bytes per 512 values with the header) fit the largest mapped region."""
+    groups = -(-n // 512)
+    return n >= 1 << 21 and -(-40 * groups // 16) * 16 + 4096 * groups <= 0xFFFFFFF0
+
+
 def run_mans(args):
     import torch
 
@@ -546,8 +554,7 @@ def run_mans(args):
     if rank == 0:
         peak, peak_src = hbm_peak()
         algo = {"map": U + M, "encode": M + C, "decode": C + M, "unmap": M + U}
-        # uint32 calls of 2 M values and more map with two kernels (the second a scan)
-        split = elem == 4 and n >= 1 << 21
+        split = elem == 4 and splits_u32_map(n)
         names = {"map": ("adm_u32_split_kernel+scan" if split else
                          "adm_u32_map_kernel" if elem == 4 else "adm_u16_map_kernel"),
                  "encode": "ans_encode_slots_kernel", "decode": "ans_decode_kernel",

@@ -227,7 +227,8 @@ mans_status compress_impl(mans_workspace* ws, mans_dtype dtype, mans_layout layo
     if (adm_u32_header_bytes(n_elems) + n_elems > ws->merged_cap) return MANS_ERR_TOO_LARGE;
     m = ws->merged;
     // Large inputs leave their records in slots for the encoder to gather, if
-    // the workspace has room for them (the default capacity does).
+    // the workspace has room for them. The default capacity does up to
+    // 531,678,720 values: a mapped region is kMaxMerged bytes at most.
     split = !map_only && n_elems >= kSplitMin && adm_u32_split_bytes(n_elems) <= ws->merged_cap;
     if (split)
       e = launch_adm_u32_split((const uint32_t*)d_in, n_elems, m, ws->group_scratch, ws->ctrl,
