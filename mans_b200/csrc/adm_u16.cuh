@@ -46,13 +46,9 @@ __host__ __device__ constexpr uint64_t u16_header_bytes(int layout, uint64_t g) 
 constexpr int kMapWarps = kAdmGroupsPerTile;  // 8
 constexpr int kMapThreads = kMapWarps * 32;   // 256
 
-// floor(a / 126) for a < 89,240: (a * ceil(2^23/126)) >> 23.
-__device__ __forceinline__ uint32_t div126(uint32_t a) {
-  return __umulhi(a << 9, 66577u);
-}
-
 // k = max(1, ceil(d/126)), code = 2r + (v <= c), r = d + 126 - 126k, i.e.
-// code = 2d + 252 + (v <= c) - 252k; (d + 125) << 9 is one multiply-add.
+// code = 2d + 252 + (v <= c) - 252k. floor(a / 126) is (a * ceil(2^23/126)) >> 23
+// for a < 89,240; (d + 125) << 9 is one multiply-add.
 __device__ __forceinline__ void adm_elem_u16(uint32_t v, uint32_t c, uint32_t& k, uint32_t& code) {
   const int s = (int)v - (int)c;
   const uint32_t d = (uint32_t)abs(s);
@@ -340,29 +336,6 @@ __device__ __forceinline__ void map16_back(const uint16_t* __restrict__ in, uint
       map16_long_lane(in, n, grp, lane, a.cnt, c, pos, L, dst, hist);
     }
   }
-}
-
-// Map group `grp` of one buffer (one warp) with a per-group look-back.
-// flags: the buffer's per-group look-back flags; msize_out: written by the
-// buffer's last group; hist: the warp's shared histogram. The group length is
-// published as soon as it is known; the prefix is read after the work that
-// does not depend on it.
-template <int kLayout = kLayoutV15>
-__device__ __forceinline__ void map16_group(const uint16_t* __restrict__ in, uint64_t n,
-                                            uint8_t* __restrict__ M, uint64_t m_cap,
-                                            unsigned long long* flags,
-                                            unsigned long long* msize_out, uint32_t grp,
-                                            uint32_t epoch, const Sink& sink, uint32_t* hist,
-                                            int lane) {
-  Map16Lane a;
-  map16_front<kLayout>(in, n, M, grp, hist, lane, a);
-  if (lane == 0) st_flag(&flags[grp], make_flag(grp == 0 ? kFlagIncl : kFlagAgg, epoch, a.L));
-  uint32_t gexcl = 0;
-  if (grp > 0) {
-    gexcl = lookback_exclusive(flags, grp, epoch, sink);
-    if (lane == 0) st_flag(&flags[grp], make_flag(kFlagIncl, epoch, gexcl + a.L));
-  }
-  map16_back<kLayout>(in, n, M, m_cap, msize_out, grp, gexcl, a, sink, hist, lane);
 }
 
 // ------------------------------------------------------------------------

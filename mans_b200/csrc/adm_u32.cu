@@ -165,7 +165,7 @@ __global__ __launch_bounds__(kMap32Threads) void adm_u32_scan_kernel(
       const uint32_t o = pre + incl[i] - v[i];
       if (k < g) {
         off[k] = o;
-        // blocks that begin inside the group's records (two at most)
+        // the block that begins inside the group's records, if any (4,096 bytes at most)
         const uint64_t a0 = rec_base + o, a1 = a0 + v[i];
         for (uint64_t b = div_up_u64(a0, kAnsBlock); b * kAnsBlock < a1; ++b) first_group[b] = (uint32_t)k;
         if (k == 0) first_group[rec_base / kAnsBlock] = 0;

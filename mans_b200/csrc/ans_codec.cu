@@ -198,8 +198,8 @@ __global__ __launch_bounds__(kEncThreads) void ans_encode_shared_kernel(
       const uint64_t s1 = ((uint64_t)b + ahead) * kAnsBlock;
       prefetch_l2(in + s1, (uint32_t)min_u64(kAnsBlock, n - s1));
     }
-    encode_block<false>(in, n, out, out_cap, out_size64, out_size32, ctrl->pdf, flags, epoch, p,
-                        sink, ss.table, ss.in[warp], bar, parity, ss.out[warp], b, lane);
+    encode_block(in, n, out, out_cap, out_size64, out_size32, ctrl->pdf, flags, epoch, p, sink,
+                 ss.table, ss.in[warp], bar, parity, ss.out[warp], b, lane);
   }
   encode_done(ctrl, epoch);
 }

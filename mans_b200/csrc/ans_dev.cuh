@@ -491,9 +491,8 @@ __device__ __forceinline__ void encode_finish(
                        pb.x, pb.sout, lane);
 }
 
-// One block as the unit of the single-pass prefix (flags per block): encode,
-// publish the aggregate, look back, store.
-template <bool kSlots>
+// One block, its words in shared memory: encode, publish the aggregate, look
+// back, store (flags per block).
 __device__ __forceinline__ void encode_block(
     const uint8_t* __restrict__ in, uint64_t n, uint8_t* __restrict__ out, uint64_t out_cap,
     unsigned long long* out_size64, uint32_t* out_size32, const uint32_t* __restrict__ pdf,
@@ -501,11 +500,11 @@ __device__ __forceinline__ void encode_block(
     uint8_t* stage, uint64_t* bar, uint32_t& parity, uint16_t* sout, uint32_t b, int lane) {
   uint32_t x;
   const uint32_t nw =
-      encode_words<!kSlots>(in, n, b, table, stage, bar, parity, sout, p, sink, lane, x);
+      encode_words<true>(in, n, b, table, stage, bar, parity, sout, p, sink, lane, x);
   const uint32_t padded = (nw + 7) & ~7u;
   if (lane == 0) st_flag(&flags[b], make_flag(b == 0 ? kFlagIncl : kFlagAgg, epoch, padded));
-  encode_finish<kSlots>(out, out_cap, n, out_size64, out_size32, pdf, flags, epoch, p, sink,
-                        EncPending{b, nw, x, sout}, lane);
+  encode_finish<false>(out, out_cap, n, out_size64, out_size32, pdf, flags, epoch, p, sink,
+                       EncPending{b, nw, x, sout}, lane);
 }
 
 // ---- decode ----

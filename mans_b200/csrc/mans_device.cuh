@@ -120,11 +120,6 @@ __device__ __forceinline__ void st_flag(unsigned long long* p, unsigned long lon
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// Prefetch one 128-byte line into L1.
-__device__ __forceinline__ void prefetch_l1(const void* p) {
-  asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
-}
-
 // Prefetch [p, p+bytes) into L2 with one bulk request (p and bytes are
 // rounded out to 16-byte boundaries; the range must lie in one allocation).
 __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
