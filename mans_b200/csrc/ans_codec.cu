@@ -123,6 +123,10 @@ __global__ __launch_bounds__(kEncMaxThreads, 1) void ans_encode_slots_kernel(
   const uint64_t n = __ldcg(&ctrl->merged_size);
   const uint64_t nb = div_up_u64(n, kAnsBlock);
   enc_fill_table(smem_raw, ctrl->enc_table, kP);
+  // Fewer blocks than warps were launched for: as many warps of every CTA as
+  // spread them evenly take part (claimed by all, the blocks crowd on the SMs
+  // that come first; 6 M small uint32 values 51.0 us a call, so 43.6).
+  const bool idle = failed || (warp >= kEncMinWarps && (uint32_t)warp * gridDim.x >= (uint32_t)nb);
   __syncthreads();
   if (!failed && nb == 0 && blockIdx.x == 0 && warp == 0)
     encode_empty(out, out_cap, kP, ctrl->pdf, out_size64, out_size32, sink, lane);
@@ -139,10 +143,6 @@ __global__ __launch_bounds__(kEncMaxThreads, 1) void ans_encode_slots_kernel(
       slots + ((uint64_t)blockIdx.x * warps + warp) * 2 * kEncSlotBytes);
   EncPending pend{0xffffffffu, 0, 0, nullptr};
   uint32_t cur = 0;
-  // Fewer blocks than warps were launched for: as many warps of every CTA as
-  // spread them evenly take part (claimed by all, the blocks crowd on the SMs
-  // that come first; 6 M small uint32 values 50.9 us a call, so 42.8).
-  const bool idle = failed || (warp >= kEncMinWarps && (uint64_t)warp * gridDim.x >= nb);
   while (!idle) {
     const uint32_t b = warp_claim(&ctrl->tile_counter[1], lane);
     if (b >= nb) break;
