@@ -169,8 +169,13 @@ __global__ __launch_bounds__(kEncMaxThreads, 1) void ans_encode_slots_kernel(
 }
 
 // The same with each block's words compacted in shared memory (no scratch in
-// global memory, no deferral), for the allocation-free call.
-__global__ __launch_bounds__(kEncThreads) void ans_encode_shared_kernel(
+// global memory, no deferral), for the allocation-free call. With a concentrated
+// symbol distribution most lanes of a step look up the same few entries, and the
+// expanded 16-byte entries save integer work; with a flat one the lanes spread
+// over many entries, and the packed 8-byte entries cost fewer shared-memory
+// wavefronts. The effective number of symbols 2^(2p) / sum(pdf^2) decides (<= 16:
+// expanded; 60 MB of two symbols at p = 10: packed 144.1 us, this 137.8).
+__global__ __launch_bounds__(kEncThreads, 2) void ans_encode_shared_kernel(
     const uint8_t* __restrict__ in, uint8_t* __restrict__ out, uint64_t out_cap,
     unsigned long long* out_size64, uint32_t* out_size32, Ctrl* ctrl,
     unsigned long long* flags, int p) {
@@ -186,7 +191,16 @@ __global__ __launch_bounds__(kEncThreads) void ans_encode_shared_kernel(
   const uint32_t epoch = *((volatile uint32_t*)&ctrl->epoch);
   const uint64_t n = __ldcg(&ctrl->merged_size);
   const uint64_t nb = div_up_u64(n, kAnsBlock);
-  if (!failed) ss.table[t] = ctrl->enc_table[t];
+  __shared__ uint32_t s_sq[kEncWarps];
+  const uint32_t q = ctrl->pdf[t], sq = __reduce_add_sync(0xffffffffu, q * q);
+  const uint2 packed = ctrl->enc_table[t];
+  if (lane == 0) s_sq[warp] = sq;
+  __syncthreads();
+  uint32_t total = 0;  // 2^22 at most
+  for (int w = 0; w < kEncWarps; ++w) total += s_sq[w];
+  const bool expanded = total * 16ull >= 1ull << (2 * p);
+  if (expanded) ss.expanded[t] = expand_enc_entry(packed, p);
+  else ss.packed[t] = packed;
   __syncthreads();
   if (!failed && nb == 0 && blockIdx.x == 0 && warp == 0)
     encode_empty(out, out_cap, p, ctrl->pdf, out_size64, out_size32, sink, lane);
@@ -198,8 +212,12 @@ __global__ __launch_bounds__(kEncThreads) void ans_encode_shared_kernel(
       const uint64_t s1 = ((uint64_t)b + ahead) * kAnsBlock;
       prefetch_l2(in + s1, (uint32_t)min_u64(kAnsBlock, n - s1));
     }
-    encode_block(in, n, out, out_cap, out_size64, out_size32, ctrl->pdf, flags, epoch, p, sink,
-                 ss.table, ss.in[warp], bar, parity, ss.out[warp], b, lane);
+    if (expanded)
+      encode_block(in, n, out, out_cap, out_size64, out_size32, ctrl->pdf, flags, epoch, p, sink,
+                   ss.expanded, ss.in[warp], bar, parity, ss.out[warp], b, lane);
+    else
+      encode_block(in, n, out, out_cap, out_size64, out_size32, ctrl->pdf, flags, epoch, p, sink,
+                   ss.packed, ss.in[warp], bar, parity, ss.out[warp], b, lane);
   }
   encode_done(ctrl, epoch);
 }

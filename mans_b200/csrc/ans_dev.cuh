@@ -35,7 +35,10 @@ __device__ __forceinline__ EncEntry4 expand_enc_entry(uint2 e, int p) {
 }
 
 struct EncSmem {  // words compacted in shared memory
-  uint2 table[kAnsSyms];  // packed entries
+  union {
+    uint2 packed[kAnsSyms];
+    EncEntry4 expanded[kAnsSyms];
+  };
   alignas(16) uint8_t in[kEncWarps][kEncStageBytes];
   uint64_t bar[kEncWarps];
   alignas(16) uint16_t out[kEncWarps][kEncOutWords];
@@ -57,14 +60,18 @@ template <int kP>
 __device__ __forceinline__ uint32_t enc_threshold(const uint2& e) {
   return ((1u << kP) - (e.y >> 20)) << (kAnsStateBits - kP);
 }
+template <int kP>
+__device__ __forceinline__ uint32_t enc_threshold(const EncEntry4& e) {
+  return e.thr;
+}
 // One interleaved step: renormalise (emit 16 bits, lanes in ascending order
 // into the compacted word buffer), then code the symbol.
 // kGuard: drop words past the buffer (see encode_words).
-template <int kP, bool kGuard, bool kShared>
+template <int kP, bool kGuard, bool kShared, typename Entry>
 __device__ __forceinline__ void enc_step(bool valid, uint32_t& x, uint32_t sym,
-                                         const uint2* __restrict__ tab, uint16_t* __restrict__ out,
+                                         const Entry* __restrict__ tab, uint16_t* __restrict__ out,
                                          uint32_t& nw, uint32_t ltmask) {
-  const uint2 e = tab[sym];
+  const Entry e = tab[sym];
   const bool wr = valid && x >= enc_threshold<kP>(e);
   const uint32_t vote = __ballot_sync(0xffffffffu, wr);
   const uint32_t idx = nw + __popc(vote & ltmask);
@@ -91,9 +98,9 @@ __device__ __forceinline__ void discard_l2_line(const void* p) {
 // The coding of one staged block (syms: the lane's first symbol in the stage,
 // bs bytes) at precision kP. kShared: sout is in shared memory (else a
 // global slot). Returns the word count; x receives the lane's final state.
-template <int kP, bool kShared>
+template <int kP, bool kShared, typename Entry>
 __device__ __forceinline__ uint32_t encode_staged(const uint8_t* syms, uint32_t bs,
-                                                  const uint2* table, uint16_t* sout, int lane,
+                                                  const Entry* table, uint16_t* sout, int lane,
                                                   uint32_t& x) {
   const uint32_t ltmask = lanemask_lt();
   x = kAnsStartState;
@@ -133,9 +140,9 @@ __device__ __forceinline__ uint32_t encode_staged(const uint8_t* syms, uint32_t 
 // interleaved coding; the word count is padded to a 16-byte multiple with
 // zeros (GpuANSEncode.h:275). Returns the number of words; x receives the
 // lane's final state.
-template <bool kSharedOut>
+template <bool kSharedOut, typename Entry>
 __device__ __forceinline__ uint32_t encode_words(const uint8_t* __restrict__ in, uint64_t n,
-                                                 uint32_t b, const uint2* table, uint8_t* stage,
+                                                 uint32_t b, const Entry* table, uint8_t* stage,
                                                  uint64_t* bar, uint32_t& parity, uint16_t* sout,
                                                  int p, const Sink& sink, int lane, uint32_t& x) {
   const uint64_t start = (uint64_t)b * kAnsBlock;
@@ -493,10 +500,11 @@ __device__ __forceinline__ void encode_finish(
 
 // One block, its words in shared memory: encode, publish the aggregate, look
 // back, store (flags per block).
+template <typename Entry>
 __device__ __forceinline__ void encode_block(
     const uint8_t* __restrict__ in, uint64_t n, uint8_t* __restrict__ out, uint64_t out_cap,
     unsigned long long* out_size64, uint32_t* out_size32, const uint32_t* __restrict__ pdf,
-    unsigned long long* flags, uint32_t epoch, int p, const Sink& sink, const uint2* table,
+    unsigned long long* flags, uint32_t epoch, int p, const Sink& sink, const Entry* table,
     uint8_t* stage, uint64_t* bar, uint32_t& parity, uint16_t* sout, uint32_t b, int lane) {
   uint32_t x;
   const uint32_t nw =

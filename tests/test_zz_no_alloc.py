@@ -92,3 +92,19 @@ def test_noalloc_encode_rejects_sizes_beyond_its_maximum():
     rc = lib.mans_ans_encode_noalloc(10, d.data_ptr(), MAX_BYTES + 1, out.data_ptr(),
                                      size.data_ptr(), torch.cuda.current_stream().cuda_stream)
     assert mb.STATUS[rc] == "MANS_ERR_TOO_LARGE"
+
+
+@pytest.mark.parametrize("p", [9, 10, 11])
+@pytest.mark.parametrize("kind", ["single", "two", "sparse", "skewed", "uniform"])
+def test_noalloc_encode_both_table_forms(oracle, kind, p):
+    """Concentrated and flat distributions take different table forms; ragged
+    sizes of a part of a block, some blocks and more blocks than warps."""
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    lib = mb.load()
+    for n in (7, 4096 * 3 - 31, 4096 * 2500 + 33):
+        x = W.random_bytes(n, n + p, kind)
+        got = _encode(lib.mans_ans_encode_noalloc, x, p)
+        assert _noalloc_status() == 0
+        np.testing.assert_array_equal(got, oracle.ans_encode(x, p))
