@@ -942,15 +942,15 @@ cudaError_t launch_batch_decompress(const BatchDev& d, uint32_t count, const uin
      (unsigned)c.ctas_per_sm[kStageDecode] * kBThreads, sizeof(BatchDecSmem), d.items, d.states,
      count, d.ctrl, chunk);
   if (marks) cudaEventRecord(marks[2], s);
-  // runs of up to 16 units, while there are 8 for every warp of a full grid, for
-  // seven eighths of them
+  // runs of up to 16 units, while there are 8 for every warp of a full grid; the
+  // last eighth of the units, and at most 16 for every warp, one by one
   auto run_of = [&](uint64_t units) {
     uint32_t r = 1;
     while (r < 16 && units >= (uint64_t)c.sms * 32 * 8 * 2 * r) r *= 2;
     return r;
   };
-  auto runs_of = [](uint64_t units, uint32_t r) {
-    return r == 1 ? 0u : (uint32_t)(units / r * 7 / 8);
+  auto runs_of = [&](uint64_t units, uint32_t r) {
+    return r == 1 ? 0u : (uint32_t)((units - min_u64(units / 8, (uint64_t)c.sms * 32 * 16)) / r);
   };
   if (groups[1]) {
     const uint32_t r = run_of(groups[1]);
