@@ -224,13 +224,15 @@ __global__ __launch_bounds__(kEncThreads, 2) void ans_encode_shared_kernel(
 
 // ------------------------------------------------------------------------
 // Decode: a warp decodes a block, or two together, from the last step to the
-// first. What bounds it: per step 22 instructions (block overhead included) of
-// which 7 go to the half-rate integer ALU, two population counts, the lookup's
-// shared-memory wavefronts, and a chain of two shared-memory loads, a vote and a
-// population count (about 130 cycles) that only other chains can hide. Two
-// kernels:
+// first. What bounds it: per step 21 to 22 instructions (24 at p = 11; block
+// overhead included) of which 7 go to the half-rate integer ALU, two population
+// counts, the lookup's shared-memory wavefronts, and a chain of two shared-memory
+// loads, a vote and a population count (about 130 cycles) that only other chains
+// can hide. Two kernels:
 //  * full: one CTA of 32 warps per SM around a replicated table of 128 KiB,
-//    pairs of blocks;
+//    pairs of blocks (CTAs of eight warps around one copy of a 4-byte table, words
+//    staged whole, took 0.575 ms on 1 GiB of detector frames, here 0.517; 1.092 on a
+//    2 GiB uint16 volume, 1.028; 131 us on 100 MB of bytes at p = 11, 95);
 //  * light: CTAs of eight warps, three to an SM, one copy of the 4-byte table,
 //    each block's words staged whole, a block per warp. Its table is built sooner,
 //    and kernels of several streams share an SM, for which the full one leaves

@@ -584,7 +584,7 @@ __global__ __launch_bounds__(32) void batch_plan_decode_kernel(const BatchItem* 
 // (two pairs of blocks per warp) where the batch has blocks enough, since the
 // CTA's barriers between chunks wait for its slowest warp; down to 8 for
 // small batches, which spreads their blocks over the SMs. (256 mixed buffers,
-// 1.6 GB: 0.985 ms; CTAs of 8 warps with one copy of a 4-byte table, 1.142.)
+// 1.6 GB: 0.959 ms; CTAs of 8 warps with one copy of a 4-byte table, 1.142.)
 // ------------------------------------------------------------------------
 struct BatchChunk {
   const uint8_t* in;  // the buffer's stream
@@ -723,9 +723,9 @@ struct BatchUnmapSmem {
 
 // Runs of up to 16 units per claim, with the buffer's fields and checks loaded
 // when a warp comes to it instead of unit by unit (256 mixed buffers, 1.6 GB:
-// 1.296 -> 1.020 ms); the last eighth of the units is claimed one by one, since a
-// unit of long lanes takes 150 us and a late run of them kept its warp alone
-// (1.015 -> 0.998 ms; 64 buffers of long lanes 9.71 -> 9.56, by units alone 9.49).
+// 1.296 -> 1.020 ms); the last units are claimed one by one, since a unit of long
+// lanes takes 150 us and a late run of them kept its warp alone (1.015 -> 0.998 ms;
+// 64 buffers of long lanes 9.71 -> 9.56, by units alone 9.49).
 // uint16 at 4 CTAs per SM (64 registers; 3 CTAs: 1.134), uint32 at 5.
 template <uint32_t kDtype>
 __global__ __launch_bounds__(kBThreads, kDtype == MANS_U16 ? 4 : 5) void batch_unmap_kernel(const BatchItem* __restrict__ items,
