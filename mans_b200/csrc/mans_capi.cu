@@ -167,9 +167,13 @@ unsigned copy_grid(const LaunchCfg& cfg, uint64_t n) {
   return (unsigned)(want < 1 ? 1 : (want < cap ? want : cap));
 }
 
-// From this many uint32 values on, a compress leaves the records in slots
-// (1 M values of detector frames: map and encode 49.3 us with the single-pass
-// map, 51.7 so; 4 M: 75 and 69; 2^28: 1,587 and 1,340).
+// From this many uint32 values on, a compress leaves the records in slots. us per
+// call, slots / single-pass map, for detector frames, Laplace codes, uniform values
+// and values within 90: 1 M values 35.7 / 34.9, 35.3 / 34.0, 44.4 / 42.8, 29.3 / 32.6;
+// 2 M 45.6 / 46.6, 44.2 / 44.7, 53.6 / 55.0, 32.9 / 39.0; 4 M 54.1 / 60.7, 58.2 /
+// 61.4, 72.9 / 78.0, 39.2 / 54.1; 2^28 1,326 / 1,579, 1,954 / 1,841, 2,680 / 2,883,
+// 610 / 1,213. (Large Laplace codes would go 6% faster the other way; the host
+// cannot tell.)
 constexpr uint64_t kSplitMin = 1u << 21;
 
 // 4 KiB blocks that n mapped elements are likely to have, for the shapes of the
